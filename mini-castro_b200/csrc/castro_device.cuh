@@ -101,6 +101,76 @@ CASTRO_HD double fminf_(double a, double b) { return (a < b) ? a : b; }
 #define DMAX(a, b) ::castro::fmaxf_((a), (b))
 #define DMIN(a, b) ::castro::fminf_((a), (b))
 
+// ---- reciprocal, quotient and square root ----
+// The step's kernels are bound by the latency of dependent FP64 chains: one
+// Riemann solve holds five reciprocals and four square roots, a corrected face
+// state one to six divisions by the same density.  The operators / and sqrt()
+// round correctly for every argument, with a test and a rare branch each, and
+// those branches keep independent chains of a thread apart.  A translation unit
+// that defines CASTRO_NR_ARITH (castro_sim.cu) takes these instead: the
+// hardware's ~20-bit seed refined by one third-order step of Newton's iteration
+// (Householder's family), straight-line, and one reciprocal for every division
+// by the same number.  Relative error at most 2^-52 (seed error below 2^-18:
+// the truncated term of rcp is e^3, of root 5/16 e^3, beyond 2^-54; then the
+// rounding of the last step and, for root, half that of x * y).  128^3 step, 2
+// species, B200: 3368 -> 2992 us (trace 459 -> 332, riemann3 790 -> 685, front
+// 370 -> 310, update 440 -> 370); 64^3, 13 species: 1027 -> 885 us; error of a
+// step against 64-bit torch unchanged (profiles of the stages in castro_sim.cu).
+// Arguments are normal numbers: the seeds flush subnormals, and a zero or an
+// infinity gives NaN where IEEE gives 0 or infinity.  Every denominator and
+// radicand here is bounded below by one of the floors above (root_floor takes
+// the floor under the root) or is a state variable that is positive by then.
+// The exact build, the per-routine kernels and the adjoint keep IEEE / and sqrt.
+#if defined(CASTRO_NR_ARITH) && !defined(CASTRO_EXACT) && defined(__CUDA_ARCH__)
+#define CASTRO_NR 1
+#else
+#define CASTRO_NR 0
+#endif
+CASTRO_HD double rcp(double x)
+{
+#if CASTRO_NR
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);          // 1/x = y / (1 - e) = y (1 + e + e^2 + ...)
+    return fma(y, fma(e, e, e), y);
+#else
+    return 1.0 / x;
+#endif
+}
+// a / b, rb = rcp(b)
+CASTRO_HD double quot(double a, double b, double rb)
+{
+#if CASTRO_NR
+    (void)b;
+    return a * rb;
+#else
+    (void)rb;
+    return a / b;
+#endif
+}
+// sqrt(x)
+CASTRO_HD double root(double x)
+{
+#if CASTRO_NR
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double g = x * y;
+    const double e = fma(-g, y, 1.0);          // sqrt(x) = g / sqrt(1 - e) = g (1 + e/2 + 3/8 e^2 + ...)
+    return fma(g * e, fma(0.375, e, 0.5), g);
+#else
+    return sqrt(x);
+#endif
+}
+// max(lo, sqrt(|x|)), lo > 0
+CASTRO_HD double root_floor(double lo, double x)
+{
+#if CASTRO_NR
+    return root(DMAX(lo * lo, fabs(x)));
+#else
+    return DMAX(lo, sqrt(fabs(x)));
+#endif
+}
+
 // ---------------------------------------------------------------------------
 // Helmholtz EOS, Source/eos.F90:141-576
 // ---------------------------------------------------------------------------
@@ -475,11 +545,12 @@ __device__ __forceinline__ void eos_eval_part(double temp, const EosConst& K, co
 
     // :491-507
     double zz = pres * deni;
-    double zzi = den / pres;
-    double chit = temp / pres * dpresdt;
+    const double presi = rcp(pres);
+    double zzi = quot(den, pres, presi);
+    double chit = quot(temp, pres, presi) * dpresdt;
     double chid = dpresdd * zzi;
     double cv = denerdt;
-    r.gam1 = chit * zz * chit / (temp * cv) + chid;
+    r.gam1 = quot(chit * zz * chit, temp * cv, rcp(temp * cv)) + chid;
     r.p = pres;
     r.e = ener;
     r.dpdT = dpresdt;
@@ -513,10 +584,10 @@ __device__ __forceinline__ EosResult eos_solve(double rho, double T, double v_wa
 {
     EosConst K;
     K.den = rho;
-    K.ytot1 = 1.0 / abar;
-    K.ye = zbar / abar;
+    K.ytot1 = rcp(abar);
+    K.ye = quot(zbar, abar, K.ytot1);
     K.din = K.ye * rho;
-    K.deni = 1.0 / rho;
+    K.deni = rcp(rho);
     K.zbar = zbar;
     DensityBasis B;
     density_basis(K.din, B);
@@ -547,7 +618,7 @@ __device__ __forceinline__ EosResult eos_solve(double rho, double T, double v_wa
         double temp_old = temp;
         double v = (MODE == EOS_RE) ? r.e : r.p;
         double dvdx = (MODE == EOS_RE) ? r.dedT : r.dpdT;
-        temp = temp - (v - v_want) / dvdx;
+        temp = temp - quot(v - v_want, dvdx, rcp(dvdx));
         temp = DMAX(0.5 * temp_old, DMIN(temp, 2.0 * temp_old));
         temp = DMAX(c_eos.mintemp, temp);
         T = temp;
@@ -573,7 +644,7 @@ __device__ __forceinline__ EosResult eos_solve(double rho, double T, double v_wa
     o.p = (MODE == EOS_RP) ? v_want : r.p;
     o.e = (MODE == EOS_RE) ? v_want : r.e;
     o.gam1 = r.gam1;
-    o.cs = sqrt(r.gam1 * r.p / rho);                                   // :556
+    o.cs = root(quot(r.gam1 * r.p, rho, K.deni));                                   // :556
     o.dedT = r.dedT;
     o.dpdT = r.dpdT;
     o.dpde = r.dpdT / r.dedT;                                          // :502-503
@@ -590,7 +661,7 @@ __device__ __forceinline__ void abar_zbar_cons(const double* u, double rhoInv, d
     for (int n = 0; n < NS; ++n) s1 = s1 + u[UFS + n] * c_net.aion_inv[n];
 #pragma unroll
     for (int n = 0; n < NS; ++n) s2 = s2 + u[UFS + n] * c_net.zion[n] * c_net.aion_inv[n];
-    abar = 1.0 / (s1 * rhoInv);
+    abar = rcp(s1 * rhoInv);
     zbar = abar * (s2 * rhoInv);
 }
 
@@ -630,14 +701,15 @@ __device__ __forceinline__ void normalize_species_pt(double* u)
     double sum = 0.0;
 #pragma unroll
     for (int n = 0; n < NS; ++n) sum = sum + u[UFS + n];
+    const double sumi = rcp(sum);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) u[UFS + n] = u[UFS + n] / sum;
+    for (int n = 0; n < NS; ++n) u[UFS + n] = quot(u[UFS + n], sum, sumi);
 }
 
 template <int NS, bool COUL>
 __device__ __forceinline__ void reset_internal_e_pt(double* u)
 {
-    double rhoInv = 1.0 / u[URHO];                                     // :196-244
+    double rhoInv = rcp(u[URHO]);                                     // :196-244
     double Up = u[UMX] * rhoInv;
     double Vp = u[UMY] * rhoInv;
     double Wp = u[UMZ] * rhoInv;
@@ -652,7 +724,12 @@ __device__ __forceinline__ void reset_internal_e_pt(double* u)
         u[UEDEN] = u[UEINT] + u[URHO] * ke;
     } else {
         double rho_eint = u[UEDEN] - u[URHO] * ke;
-        if (rho_eint > 0.0 && rho_eint / u[UEDEN] > dual_energy_eta2) {
+#if CASTRO_NR
+        const bool thermal = rho_eint > dual_energy_eta2 * u[UEDEN];
+#else
+        const bool thermal = rho_eint / u[UEDEN] > dual_energy_eta2;
+#endif
+        if (rho_eint > 0.0 && thermal) {
             u[UEINT] = rho_eint;
         } else if (u[UEINT] <= 0.0) {
             double abar, zbar;
@@ -666,7 +743,7 @@ __device__ __forceinline__ void reset_internal_e_pt(double* u)
 template <int NS, bool COUL>
 __device__ __forceinline__ void compute_temp_pt(double* u)
 {
-    double rhoInv = 1.0 / u[URHO];                                     // :280-291
+    double rhoInv = rcp(u[URHO]);                                     // :280-291
     double abar, zbar;
     abar_zbar_cons<NS>(u, rhoInv, abar, zbar);
     EosResult r = eos_solve<EOS_RE, COUL, false>(u[URHO], u[UTEMP], u[UEINT] * rhoInv, abar, zbar);   // reads T only
@@ -688,7 +765,7 @@ __device__ __forceinline__ void clean_state_pt(double* u)
 template <int NS, bool COUL>
 __device__ __forceinline__ double estdt_pt(const double* u, double dx0, double dx1, double dx2)
 {
-    double rhoInv = 1.0 / u[URHO];
+    double rhoInv = rcp(u[URHO]);
     double abar, zbar;
     abar_zbar_cons<NS>(u, rhoInv, abar, zbar);
     EosResult r = eos_solve<EOS_RE, COUL>(u[URHO], u[UTEMP], u[UEINT] * rhoInv, abar, zbar);
@@ -696,9 +773,9 @@ __device__ __forceinline__ double estdt_pt(const double* u, double dx0, double d
     double uy = u[UMY] * rhoInv;
     double uz = u[UMZ] * rhoInv;
     double c = r.cs;
-    double dt1 = dx0 / (c + fabs(ux));
-    double dt2 = dx1 / (c + fabs(uy));
-    double dt3 = dx2 / (c + fabs(uz));
+    double dt1 = quot(dx0, c + fabs(ux), rcp(c + fabs(ux)));
+    double dt2 = quot(dx1, c + fabs(uy), rcp(c + fabs(uy)));
+    double dt3 = quot(dx2, c + fabs(uz), rcp(c + fabs(uz)));
     return DMIN(DMIN(dt1, dt2), dt3);
 }
 
@@ -708,12 +785,20 @@ template <int NS, bool COUL>
 __device__ __forceinline__ void ctoprim_pt(const double* u, double* q, double* qaux)
 {
     q[QRHO] = u[URHO];
-    double rhoinv = 1.0 / q[QRHO];
+    double rhoinv = rcp(q[QRHO]);
     q[QU] = u[UMX] * rhoinv;
     q[QV] = u[UMY] * rhoinv;
     q[QW] = u[UMZ] * rhoinv;
     double kineng = 0.5 * q[QRHO] * (q[QU] * q[QU] + q[QV] * q[QV] + q[QW] * q[QW]);
-    if ((u[UEDEN] - kineng) / u[UEDEN] > dual_energy_eta1)
+#if CASTRO_NR
+    // the quotient above 1, without the division
+    static_assert(dual_energy_eta1 == 1.0, "the comparison below is the quotient's against 1");
+    const double eth = u[UEDEN] - kineng, etot = u[UEDEN];
+    const bool thermal = etot > 0.0 ? eth > etot : etot < 0.0 ? eth < etot : eth > 0.0;
+#else
+    const bool thermal = (u[UEDEN] - kineng) / u[UEDEN] > dual_energy_eta1;
+#endif
+    if (thermal)
         q[QREINT] = (u[UEDEN] - kineng) * rhoinv;
     else
         q[QREINT] = u[UEINT] * rhoinv;
@@ -725,7 +810,7 @@ __device__ __forceinline__ void ctoprim_pt(const double* u, double* q, double* q
     for (int n = 0; n < NS; ++n) s1 = s1 + q[QFS + n] * c_net.aion_inv[n];
 #pragma unroll
     for (int n = 0; n < NS; ++n) s2 = s2 + q[QFS + n] * c_net.zion[n] * c_net.aion_inv[n];
-    double abar = 1.0 / s1;
+    double abar = rcp(s1);
     double zbar = abar * s2;
     EosResult r = eos_solve<EOS_RE, COUL>(q[QRHO], q[QTEMP], q[QREINT], abar, zbar);
     q[QTEMP] = r.T;
@@ -763,7 +848,7 @@ CASTRO_HD double uflatten(const L& ld, int i, int j, int k)
         double dp = pr - pl;
         int s = (dp > 0.0) ? -1 : 1;   // s = -ishft
         double denom = DMAX(small_pres, fabs(dp2));
-        double denominv = 1.0 / denom;
+        double denominv = rcp(denom);
         double zeta = fabs(dp) * denominv;
         double z = DMIN(1.0, DMAX(0.0, dzcut * (zeta - zcut1)));
         double tst = (du <= 0.0) ? 1.0 : 0.0;
@@ -778,7 +863,7 @@ CASTRO_HD double uflatten(const L& ld, int i, int j, int k)
            - ld.q(i + (s - 1) * ex, j + (s - 1) * ey, k + (s - 1) * ez, qun);
         dp = pr - pl;
         denom = DMAX(small_pres, fabs(dp2));
-        denominv = 1.0 / denom;
+        denominv = rcp(denom);
         zeta = fabs(dp) * denominv;
         double z2 = DMIN(1.0, DMAX(0.0, dzcut * (zeta - zcut1)));
         tst = (du <= 0.0) ? 1.0 : 0.0;
@@ -868,11 +953,12 @@ CASTRO_HD void trace_project(const double I[3][4], double gam_g_ref, double un, 
     double p_ref = I[wr][2];
     double rhoe_g_ref = I[wr][3];
     rho_ref = DMAX(rho_ref, small_dens);
-    double rho_ref_inv = 1.0 / rho_ref;
+    double rho_ref_inv = rcp(rho_ref);
     p_ref = DMAX(p_ref, small_pres);
     double csq_ref = gam_g_ref * p_ref * rho_ref_inv;
-    double cc_ref = sqrt(csq_ref);
-    double cc_ref_inv = 1.0 / cc_ref;
+    double cc_ref = root(csq_ref);
+    double cc_ref_inv = rcp(cc_ref);
+    double csq_ref_inv = rcp(csq_ref);
     double h_g_ref = (p_ref + rhoe_g_ref) * rho_ref_inv;
     double dum = un_ref - I[0][1];
     double dptotm = p_ref - I[0][2];
@@ -883,8 +969,8 @@ CASTRO_HD void trace_project(const double I[3][4], double gam_g_ref, double un, 
     double dptotp = p_ref - I[2][2];
     double alpham = 0.5 * (dptotm * rho_ref_inv * cc_ref_inv - dum) * rho_ref * cc_ref_inv;
     double alphap = 0.5 * (dptotp * rho_ref_inv * cc_ref_inv + dup) * rho_ref * cc_ref_inv;
-    double alpha0r = drho - dptot / csq_ref;
-    double alpha0e_g = drhoe_g - dptot * h_g_ref / csq_ref;
+    double alpha0r = drho - quot(dptot, csq_ref, csq_ref_inv);
+    double alpha0e_g = drhoe_g - quot(dptot * h_g_ref, csq_ref, csq_ref_inv);
     if (plus) {
         alpham = (un - cc > 0.0) ? 0.0 : -alpham;
         alphap = (un + cc > 0.0) ? 0.0 : -alphap;
@@ -1016,9 +1102,9 @@ CASTRO_HD void riemann_cgf(const double* ql, const double* qr, double gamcl, dou
     double csmall = DMAX(small, small * DMAX(cr, cl));
     double cavg = 0.5 * (cr + cl);
     double wsmall = small_dens * csmall;
-    double wl = DMAX(wsmall, sqrt(fabs(gamcl * pl * rl)));
-    double wr = DMAX(wsmall, sqrt(fabs(gamcr * pr * rr)));
-    double wwinv = 1.0 / (wl + wr);
+    double wl = root_floor(wsmall, gamcl * pl * rl);
+    double wr = root_floor(wsmall, gamcr * pr * rr);
+    double wwinv = rcp(wl + wr);
     double pstar = ((wr * pl + wl * pr) + wl * wr * (ul - ur)) * wwinv;
     double ustar = ((wl * ul + wr * ur) + (pl - pr)) * wwinv;
     pstar = DMAX(pstar, small_pres);
@@ -1034,21 +1120,19 @@ CASTRO_HD void riemann_cgf(const double* ql, const double* qr, double gamcl, dou
     double reo = fp * rel + fm * rer;
     double gamco = fp * gamcl + fm * gamcr;
     ro = DMAX(small_dens, ro);
-    double roinv = 1.0 / ro;
-    double co = sqrt(fabs(gamco * po * roinv));
-    co = DMAX(csmall, co);
-    double co2inv = 1.0 / (co * co);
+    double roinv = rcp(ro);
+    double co = root_floor(csmall, gamco * po * roinv);
+    double co2inv = rcp(co * co);
     double qv1 = fp * v1l + fm * v1r;
     double qv2 = fp * v2l + fm * v2r;
 
     double drho = (pstar - po) * co2inv;
     double rstar = ro + drho;
     rstar = DMAX(small_dens, rstar);
-    double rstarinv = 1.0 / rstar;
+    double rstarinv = rcp(rstar);
     double entho = (reo + po) * roinv * co2inv;
     double estar = reo + (pstar - po) * entho;
-    double cstar = sqrt(fabs(gamco * pstar * rstarinv));
-    cstar = DMAX(cstar, csmall);
+    double cstar = root_floor(csmall, gamco * pstar * rstarinv);
 
     sgnm = copysign(1.0, ustar);                                       // riemann.F90:225 (no zero guard)
     double spout = co - sgnm * uo;
@@ -1056,7 +1140,7 @@ CASTRO_HD void riemann_cgf(const double* ql, const double* qr, double gamcl, dou
     double ushock = 0.5 * (spin + spout);
     if (pstar - po > 0.0) { spin = ushock; spout = ushock; }
     double scr = (spout - spin == 0.0) ? small * cavg : spout - spin;
-    double scrinv = 1.0 / scr;
+    double scrinv = rcp(scr);
     double frac = (1.0 + (spout + spin) * scrinv) * 0.5;
     frac = DMAX(0.0, DMIN(1.0, frac));
 
@@ -1066,7 +1150,7 @@ CASTRO_HD void riemann_cgf(const double* ql, const double* qr, double gamcl, dou
     double regdnv = frac * estar + (1.0 - frac) * reo;
     if (spout < 0.0) { qrho = ro; qu = uo; qp = po; regdnv = reo; }
     if (spin >= 0.0) { qrho = rstar; qu = ustar; qp = pstar; regdnv = estar; }
-    double regdnvinv = 1.0 / regdnv;
+    double regdnvinv = rcp(regdnv);
     double qgame = qp * regdnvinv + 1.0;
     qp = DMAX(qp, small_pres);
 
@@ -1130,11 +1214,12 @@ CASTRO_HD bool trans1_state(const double* lq, const double* fr, const double* fl
                                              double cdtdx, double* lqo)
 {
     using R = TF<NS>;
+    const double rrnew = lq[SRHO] - cdtdx * (fr[R::RHO] - fl[R::RHO]);
+    const double rrnewinv = rcp(rrnew);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
-        double rrnew = lq[SRHO] - cdtdx * (fr[R::RHO] - fl[R::RHO]);
         double compu = lq[SRHO] * lq[SX + n] - cdtdx * (fr[R::X + n] - fl[R::X + n]);
-        lqo[SX + n] = compu / rrnew;
+        lqo[SX + n] = quot(compu, rrnew, rrnewinv);
     }
     double pgp = fr[R::PG], pgm = fl[R::PG];
     double ugp = fr[R::UG], ugm = fl[R::UG];
@@ -1148,7 +1233,8 @@ CASTRO_HD bool trans1_state(const double* lq, const double* fr, const double* fl
     double rwl2 = rrl2 * lq[SW];
     double ekenl2 = 0.5 * rrl2 * (lq[SU] * lq[SU] + lq[SV] * lq[SV] + lq[SW] * lq[SW]);
     double rel2 = lq[SREI] + ekenl2;
-    double rrnewl2 = rrl2 - cdtdx * (fr[R::RHO] - fl[R::RHO]);
+    double rrnewl2 = rrnew;
+    double rhoinv = rrnewinv;
     double runewl2 = rul2 - cdtdx * (fr[R::MX] - fl[R::MX]);
     double rvnewl2 = rvl2 - cdtdx * (fr[R::MY] - fl[R::MY]);
     double rwnewl2 = rwl2 - cdtdx * (fr[R::MZ] - fl[R::MZ]);
@@ -1156,10 +1242,10 @@ CASTRO_HD bool trans1_state(const double* lq, const double* fr, const double* fl
     bool reset_state = false;
     if (rrnewl2 < 0.0) {
         rrnewl2 = rrl2; runewl2 = rul2; rvnewl2 = rvl2; rwnewl2 = rwl2; renewl2 = rel2;
+        rhoinv = rcp(rrnewl2);
         reset_state = true;
     }
     lqo[SRHO] = rrnewl2;
-    double rhoinv = 1.0 / rrnewl2;
     lqo[SU] = runewl2 * rhoinv;
     lqo[SV] = rvnewl2 * rhoinv;
     lqo[SW] = rwnewl2 * rhoinv;
@@ -1183,13 +1269,13 @@ CASTRO_HD bool trans2_state(const double* lq, const double* f2r, const double* f
                                              double cdtdx2, double cdtdx3, double* lqo)
 {
     using R = TF<NS>;
+    const double rrnew = lq[SRHO] - cdtdx2 * (f2r[R::RHO] - f2l[R::RHO]) - cdtdx3 * (f3r[R::RHO] - f3l[R::RHO]);
+    double rinv = rcp(rrnew);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
-        double rrr = lq[SRHO];
-        double compr = rrr * lq[SX + n];
-        double rrnewr = rrr - cdtdx2 * (f2r[R::RHO] - f2l[R::RHO]) - cdtdx3 * (f3r[R::RHO] - f3l[R::RHO]);
+        double compr = lq[SRHO] * lq[SX + n];
         double compnr = compr - cdtdx2 * (f2r[R::X + n] - f2l[R::X + n]) - cdtdx3 * (f3r[R::X + n] - f3l[R::X + n]);
-        lqo[SX + n] = compnr / rrnewr;
+        lqo[SX + n] = quot(compnr, rrnew, rinv);
     }
     double pg2p = f2r[R::PG], pg2m = f2l[R::PG], ug2p = f2r[R::UG], ug2m = f2l[R::UG];
     double du2p = pg2p * ug2p - pg2m * ug2m;
@@ -1208,7 +1294,7 @@ CASTRO_HD bool trans2_state(const double* lq, const double* f2r, const double* f
     double rwr = rrr * lq[SW];
     double ekenr = 0.5 * rrr * (lq[SU] * lq[SU] + lq[SV] * lq[SV] + lq[SW] * lq[SW]);
     double rer = lq[SREI] + ekenr;
-    double rrnewr = rrr - cdtdx2 * (f2r[R::RHO] - f2l[R::RHO]) - cdtdx3 * (f3r[R::RHO] - f3l[R::RHO]);
+    double rrnewr = rrnew;
     double runewr = rur - cdtdx2 * (f2r[R::MX] - f2l[R::MX]) - cdtdx3 * (f3r[R::MX] - f3l[R::MX]);
     double rvnewr = rvr - cdtdx2 * (f2r[R::MY] - f2l[R::MY]) - cdtdx3 * (f3r[R::MY] - f3l[R::MY]);
     double rwnewr = rwr - cdtdx2 * (f2r[R::MZ] - f2l[R::MZ]) - cdtdx3 * (f3r[R::MZ] - f3l[R::MZ]);
@@ -1216,13 +1302,14 @@ CASTRO_HD bool trans2_state(const double* lq, const double* f2r, const double* f
     bool reset_state = false;
     if (rrnewr < 0.0) {
         rrnewr = rrr; runewr = rur; rvnewr = rvr; rwnewr = rwr; renewr = rer;
+        rinv = rcp(rrnewr);
         reset_state = true;
     }
     lqo[SRHO] = rrnewr;
-    lqo[SU] = runewr / rrnewr;
-    lqo[SV] = rvnewr / rrnewr;
-    lqo[SW] = rwnewr / rrnewr;
-    double rhoekenr = 0.5 * (runewr * runewr + rvnewr * rvnewr + rwnewr * rwnewr) / rrnewr;
+    lqo[SU] = quot(runewr, rrnewr, rinv);
+    lqo[SV] = quot(rvnewr, rrnewr, rinv);
+    lqo[SW] = quot(rwnewr, rrnewr, rinv);
+    double rhoekenr = quot(0.5 * (runewr * runewr + rvnewr * rvnewr + rwnewr * rwnewr), rrnewr, rinv);
     lqo[SREI] = renewr - rhoekenr;
     lqo[SPRES] = reset_state ? lq[SPRES] : lq[SPRES] - p2new - p3new;
     lqo[SPRES] = DMAX(lqo[SPRES], small_pres);

@@ -38,6 +38,7 @@
 #include <string>
 #include <vector>
 
+#define CASTRO_NR_ARITH   // refined reciprocals and square roots in the production build (castro_device.cuh)
 #include "castro_common.cuh"
 #include "../../include/castro_b200.h"
 
