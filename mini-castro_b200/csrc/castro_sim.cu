@@ -147,13 +147,26 @@ struct InstState {
     int steps, pad;
 };
 
-struct Work { int box, sub, start, count; };
+// Work item: the points [start, start + count) of a region in x-fastest order.
+// i0, j0, k0: the first point relative to the region's low corner; mx, my: the
+// multipliers of div_small for the region's x and y extents, so that a thread
+// finds its point with two multiplications.
+struct Work {
+    int box, sub, count;
+    int i0, j0, k0;
+    unsigned mx, my;
+};
 
 enum Region { R_VALID = 0, R_G1, R_G4, R_TBX, R_EBX, R_GHOST, R_SEG };
 
+// Points of a region are numbered in 32 bits (castro_sim_create rejects a
+// domain with a region of 2^31 points or more), components by 64-bit plane
+// offsets: one multiply-add per address, where 64-bit point numbers cost four
+// to six integer instructions for every double loaded or stored.
 struct Reg {
     int lx, ly, lz, nx, ny, nz;
-    long long np;
+    unsigned np;
+    __device__ __forceinline__ size_t plane(unsigned c) const { return (size_t)np * c; }   // offset of component c
 };
 
 __host__ __device__ __forceinline__ Reg make_reg(const int* lo, const int* hi, int kind, int sub)
@@ -189,13 +202,55 @@ __host__ __device__ __forceinline__ Reg make_reg(const int* lo, const int* hi, i
     Reg r;
     r.lx = l[0]; r.ly = l[1]; r.lz = l[2];
     r.nx = h[0] - l[0] + 1; r.ny = h[1] - l[1] + 1; r.nz = h[2] - l[2] + 1;
-    r.np = (long long)r.nx * r.ny * r.nz;
+    r.np = (unsigned)r.nx * (unsigned)r.ny * (unsigned)r.nz;
     return r;
 }
 
-__device__ __forceinline__ long long ridx(const Reg& r, int i, int j, int k)
+__device__ __forceinline__ int ridx(const Reg& r, int i, int j, int k)
 {
-    return (long long)(i - r.lx) + (long long)r.nx * ((long long)(j - r.ly) + (long long)r.ny * (k - r.lz));
+    return (i - r.lx) + r.nx * ((j - r.ly) + r.ny * (k - r.lz));
+}
+
+// A thread's point by two 32-bit multiplications (the 64-bit % and / by the
+// region's extents were ~150 instructions of every thread).  With the 32-bit
+// point numbers above, 128^3 step, 2 species, B200: front 310 -> 290 us, prep
+// 90 -> 84, riemann1 259 -> 233, riemann2 682 -> 654.
+// t / n for t < n + MAX_ITEM, m = div_mult(n): floor(2^32 / n) + 1 gives the
+// quotient exactly while t n < 2^32; beyond n = 2^15 the quotient is 0 or 1
+constexpr int MAX_ITEM = 1024;
+__host__ __device__ __forceinline__ unsigned div_mult(int n)
+{
+    return (n == 1 || n > 32768) ? 0u : (unsigned)(4294967296ull / (unsigned)n) + 1u;
+}
+__device__ __forceinline__ int div_small(int t, int n, unsigned m)
+{
+    if (m) return (int)__umulhi((unsigned)t, m);
+    return n == 1 ? t : (int)(t >= n);
+}
+
+__host__ __device__ __forceinline__ Work make_work(int box, int sub, long long start, int count, const Reg& R)
+{
+    Work w;
+    w.box = box;
+    w.sub = sub;
+    w.count = count;
+    w.i0 = (int)(start % R.nx);
+    const long long t = start / R.nx;
+    w.j0 = (int)(t % R.ny);
+    w.k0 = (int)(t / R.ny);
+    w.mx = div_mult(R.nx);
+    w.my = div_mult(R.ny);
+    return w;
+}
+
+// point tp of item w, a point of region R
+__device__ __forceinline__ void item_point(const Work& w, const Reg& R, int tp, int& i, int& j, int& k)
+{
+    const int t = w.i0 + tp, q = div_small(t, R.nx, w.mx);
+    const int u = w.j0 + q, r = div_small(u, R.ny, w.my);
+    i = R.lx + t - q * R.nx;
+    j = R.ly + u - r * R.ny;
+    k = R.lz + w.k0 + r;
 }
 
 struct SimDev {
@@ -228,11 +283,7 @@ __device__ __forceinline__ bool work_point_rep(const Work& w, const SimDev& S, i
     int rs = sub;
     if (kind == R_TBX && subkind_tbx == 0) rs = 4 * sub;   // tbx[d][d]
     R = make_reg(B.lo, B.hi, kind, rs);
-    long long t = (long long)w.start + tp;
-    i = R.lx + (int)(t % R.nx);
-    long long t2 = t / R.nx;
-    j = R.ly + (int)(t2 % R.ny);
-    k = R.lz + (int)(t2 / R.ny);
+    item_point(w, R, tp, i, j, k);
     return true;
 }
 
@@ -260,7 +311,7 @@ template <int NS>
 struct QLoader {
     const double* base;
     Reg R;
-    __device__ __forceinline__ double at(int i, int j, int k, int c) const { return base[ridx(R, i, j, k) + R.np * c]; }
+    __device__ __forceinline__ double at(int i, int j, int k, int c) const { return (base + ridx(R, i, j, k))[R.plane(c)]; }
     __device__ __forceinline__ double q(int i, int j, int k, int n) const
     {
         int c = (n == QRHO) ? QF<NS>::RHO : (n <= QW) ? n : (n == QPRES) ? QF<NS>::P : (n == QREINT) ? QF<NS>::RE : QF<NS>::X + (n - QFS);
@@ -313,35 +364,35 @@ __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
     constexpr int NVAR = Dims<NS>::NVAR, QVAR = Dims<NS>::QVAR;
     double u[NVAR];
     double* U = S.U + B.offU;
-    long long id = ridx(R, i, j, k);
+    const int id = ridx(R, i, j, k);
 #pragma unroll
-    for (int n = 0; n < NVAR; ++n) u[n] = U[id + R.np * n];
+    for (int n = 0; n < NVAR; ++n) u[n] = (U + id)[R.plane(n)];
     clean_state_pt<NS, COUL>(u);                    // Castro_advance.cpp:51
 #pragma unroll
-    for (int n = 0; n < NVAR; ++n) U[id + R.np * n] = u[n];
+    for (int n = 0; n < NVAR; ++n) (U + id)[R.plane(n)] = u[n];
     clean_state_pt<NS, COUL>(u);                    // Castro_advance.cpp:66 (valid part of Sborder)
     const InstDev& I = S.inst[B.inst];
     const Reg R1 = u_region(I);
     double* Ub = S.Ub + B.offUb;
-    long long id1 = ridx(R1, i, j, k);
+    const int id1 = ridx(R1, i, j, k);
 #pragma unroll
-    for (int n = 0; n < NVAR; ++n) Ub[id1 + R1.np * n] = u[n];
+    for (int n = 0; n < NVAR; ++n) (Ub + id1)[R1.plane(n)] = u[n];
     double q[QVAR], qa[NQAUX];
     ctoprim_pt<NS, COUL>(u, q, qa);                 // Castro_hydro.cpp:64-70
     const Reg R4 = q_region(I);
     double* Q = S.Q + B.offQ;
-    long long id4 = ridx(R4, i, j, k);
+    const int id4 = ridx(R4, i, j, k);
     using F = QF<NS>;
-    Q[id4 + R4.np * F::RHO] = q[QRHO];
-    Q[id4 + R4.np * (F::U + 0)] = q[QU];
-    Q[id4 + R4.np * (F::U + 1)] = q[QV];
-    Q[id4 + R4.np * (F::U + 2)] = q[QW];
-    Q[id4 + R4.np * F::P] = q[QPRES];
-    Q[id4 + R4.np * F::RE] = q[QREINT];
+    (Q + id4)[R4.plane(F::RHO)] = q[QRHO];
+    (Q + id4)[R4.plane(F::U + 0)] = q[QU];
+    (Q + id4)[R4.plane(F::U + 1)] = q[QV];
+    (Q + id4)[R4.plane(F::U + 2)] = q[QW];
+    (Q + id4)[R4.plane(F::P)] = q[QPRES];
+    (Q + id4)[R4.plane(F::RE)] = q[QREINT];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) Q[id4 + R4.np * (F::X + n)] = q[QFS + n];
-    Q[id4 + R4.np * F::GAMC] = qa[QGAMC];
-    Q[id4 + R4.np * F::C] = qa[QC];
+    for (int n = 0; n < NS; ++n) (Q + id4)[R4.plane(F::X + n)] = q[QFS + n];
+    (Q + id4)[R4.plane(F::GAMC)] = qa[QGAMC];
+    (Q + id4)[R4.plane(F::C)] = qa[QC];
 }
 
 template <int NS, bool COUL>
@@ -373,26 +424,23 @@ __device__ __forceinline__ void ghost_body(const SimDev& S, const Work& w)
     const BoxDev& B = S.boxes[w.box];
     const InstDev& I = S.inst[B.inst];
     const Reg RS = make_reg(I.dom_lo, I.dom_hi, R_GHOST, w.sub);
-    const long long t = (long long)w.start + threadIdx.x;
-    const int i = RS.lx + (int)(t % RS.nx);
-    const long long t2 = t / RS.nx;
-    const int j = RS.ly + (int)(t2 % RS.ny);
-    const int k = RS.lz + (int)(t2 / RS.ny);
+    int i, j, k;
+    item_point(w, RS, threadIdx.x, i, j, k);
     const int ii = map_bc(i, I.dom_lo[0], I.dom_hi[0], I.bc);
     const int jj = map_bc(j, I.dom_lo[1], I.dom_hi[1], I.bc);
     const int kk = map_bc(k, I.dom_lo[2], I.dom_hi[2], I.bc);
     const Reg R = q_region(I);
     double* Q = S.Q + B.offQ;
-    const long long is = ridx(R, ii, jj, kk), id = ridx(R, i, j, k);
+    const int is = ridx(R, ii, jj, kk), id = ridx(R, i, j, k);
 #pragma unroll
-    for (int c = 0; c < QF<NS>::N; ++c) Q[id + R.np * c] = Q[is + R.np * c];
+    for (int c = 0; c < QF<NS>::N; ++c) (Q + id)[R.plane(c)] = (Q + is)[R.plane(c)];
     if (i >= I.dom_lo[0] - 1 && i <= I.dom_hi[0] + 1 && j >= I.dom_lo[1] - 1 && j <= I.dom_hi[1] + 1 &&
         k >= I.dom_lo[2] - 1 && k <= I.dom_hi[2] + 1) {
         const Reg R1 = u_region(I);
         double* Ub = S.Ub + B.offUb;
-        const long long is1 = ridx(R1, ii, jj, kk), id1 = ridx(R1, i, j, k);
+        const int is1 = ridx(R1, ii, jj, kk), id1 = ridx(R1, i, j, k);
 #pragma unroll
-        for (int n = 0; n < Dims<NS>::NVAR; ++n) Ub[id1 + R1.np * n] = Ub[is1 + R1.np * n];
+        for (int n = 0; n < Dims<NS>::NVAR; ++n) (Ub + id1)[R1.plane(n)] = (Ub + is1)[R1.plane(n)];
     }
 }
 
@@ -430,7 +478,7 @@ __device__ __forceinline__ void prep_body(const SimDev& S, const Work& w)
                         + Qv(i, j - 1, k, 2) - Qv(i, j - 1, k - 1, 2)
                         + Qv(i - 1, j, k, 2) - Qv(i - 1, j, k - 1, 2)
                         + Qv(i - 1, j - 1, k, 2) - Qv(i - 1, j - 1, k - 1, 2)) * dzinv;
-    long long id = ridx(R, i, j, k);
+    const int id = ridx(R, i, j, k);
     S.Div[B.offDiv + id] = ux + vy + wz;
     S.Div[B.offDiv + id + R.np] = uflatten(ld, i, j, k);
 }
@@ -471,13 +519,12 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
     double* Tr = S.Tr + B.offTr[D];
     // linear indices of zone z0 (Q, flatn) and of its low face (face states);
     // the face of zone lo-1 lies one stride below tbx[D][D] and is never stored
-    const long long q0 = ridx(R4, p[0], p[1], p[2]);
-    const long long f0 = ridx(R1, p[0], p[1], p[2]);
-    const long long t0 = ridx(RT, p[0], p[1], p[2]);
-    const long long sq = D == 0 ? 1 : D == 1 ? (long long)R4.nx : (long long)R4.nx * R4.ny;
-    const long long sf = D == 0 ? 1 : D == 1 ? (long long)R1.nx : (long long)R1.nx * R1.ny;
-    const long long st = D == 0 ? 1 : D == 1 ? (long long)RT.nx : (long long)RT.nx * RT.ny;
-    const long long nq = R4.np, nt = RT.np;
+    const int q0 = ridx(R4, p[0], p[1], p[2]);
+    const int f0 = ridx(R1, p[0], p[1], p[2]);
+    const int t0 = ridx(RT, p[0], p[1], p[2]);
+    const int sq = D == 0 ? 1 : D == 1 ? R4.nx : R4.nx * R4.ny;
+    const int sf = D == 0 ? 1 : D == 1 ? R1.nx : R1.nx * R1.ny;
+    const int st = D == 0 ? 1 : D == 1 ? RT.nx : RT.nx * RT.ny;
 
     // pass 1: rho, u_D, p, rhoe, gamma_c.  Window of variable v at zone z:
     // wa = s(z), wb = s(z+1), wd = slope(z), we = edge(z) (minus edge of z).
@@ -490,7 +537,7 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
     double wa[NW], wb[NW], wd[NW], we[NW], nxt[NW];
 #pragma unroll
     for (int v = 0; v < NW; ++v) {
-        const double* c = Q + q0 + (long long)cw[v] * nq;
+        const double* c = Q + q0 + R4.plane(cw[v]);
         double sm2 = c[-2 * sq], sm1 = c[-sq], s0 = c[0], sp1 = c[sq];
         nxt[v] = c[2 * sq];
         double dm = vl_slope(sm2, sm1, s0);
@@ -499,7 +546,7 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
         wa[v] = s0;
         wb[v] = sp1;
     }
-    double flatn_n = Fl[f0], cc_n = Q[q0 + (long long)F::C * nq];
+    double flatn_n = Fl[f0], cc_n = (Q + q0)[R4.plane(F::C)];
 #pragma unroll 1
     for (int z = 0; z < n; ++z) {
         const double flatn = flatn_n;
@@ -509,9 +556,9 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
 #pragma unroll
         for (int v = 0; v < NW; ++v) {
             cur[v] = nxt[v];
-            nxt[v] = Q[q0 + (z + 3) * sq + (long long)cw[v] * nq];
+            nxt[v] = (Q + (q0 + (z + 3) * sq))[R4.plane(cw[v])];
         }
-        cc_n = Q[q0 + (z + 1) * sq + (long long)F::C * nq];
+        cc_n = (Q + (q0 + (z + 1) * sq))[R4.plane(F::C)];
         if (z + 1 < n) flatn_n = Fl[f0 + (z + 1) * sf];
         double Ip[3][4], Im[3][4], gp0, gm0, gp2, gm2;
 #pragma unroll
@@ -539,19 +586,19 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
             double r, u, re, pr;
             trace_project(Im, gm0, un, cc, true, r, u, re, pr);
             double* t = Tr + (t0 + z * st);
-            t[nt * (NQS + SRHO)] = r;
-            t[nt * (NQS + SU + D)] = u;
-            t[nt * (NQS + SREI)] = re;
-            t[nt * (NQS + SPRES)] = pr;
+            t[RT.plane(NQS + SRHO)] = r;
+            t[RT.plane(NQS + SU + D)] = u;
+            t[RT.plane(NQS + SREI)] = re;
+            t[RT.plane(NQS + SPRES)] = pr;
         }
         if (z <= zhi) {
             double r, u, re, pr;
             trace_project(Ip, gp2, un, cc, false, r, u, re, pr);
             double* t = Tr + (t0 + (z + 1) * st);
-            t[nt * SRHO] = r;
-            t[nt * (SU + D)] = u;
-            t[nt * SREI] = re;
-            t[nt * SPRES] = pr;
+            t[RT.plane(SRHO)] = r;
+            t[RT.plane(SU + D)] = u;
+            t[RT.plane(SREI)] = re;
+            t[RT.plane(SPRES)] = pr;
         }
     }
 
@@ -563,8 +610,8 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
     for (int v = 0; v < 2 + NS; ++v) {
         const int comp = v == 0 ? F::U + T1 : v == 1 ? F::U + T2 : F::X + (v - 2);
         const int slot = v == 0 ? SU + T1 : v == 1 ? SU + T2 : SX + (v - 2);
-        const double* c = Q + q0 + (long long)comp * nq;
-        const double* cu = Q + q0 + (long long)(F::U + D) * nq;
+        const double* c = Q + q0 + R4.plane(comp);
+        const double* cu = Q + q0 + R4.plane(F::U + D);
         double sm2 = c[-2 * sq], sm1 = c[-sq], a = c[0], bq = c[sq];
         double nxt2 = c[2 * sq], un_n = cu[0], flatn_n2 = Fl[f0];
         double d = vl_slope(sm1, a, bq);
@@ -584,8 +631,8 @@ __device__ __forceinline__ void trace_segment(const SimDev& S, const BoxDev& B, 
             const double s6 = 6.0 * a - 3.0 * (sm + sp);
             double ip, im;
             ppm_int_wave(sm, sp, s6, un, dtdx, ip, im);
-            if (z >= zlo) Tr[t0 + z * st + nt * (NQS + slot)] = im;
-            if (z <= zhi) Tr[t0 + (z + 1) * st + nt * slot] = ip;
+            if (z >= zlo) (Tr + (t0 + z * st))[RT.plane(NQS + slot)] = im;
+            if (z <= zhi) (Tr + (t0 + (z + 1) * st))[RT.plane(slot)] = ip;
             a = bq;
             bq = s2;
             d = dn;
@@ -646,25 +693,25 @@ __device__ __forceinline__ double2 riemann_at(const QLoader<NS>& ld, int i, int 
 }
 
 template <int NS>
-__device__ __forceinline__ void store_tf(double* base, const Reg& R, long long f, const double* flx, double pg, double ug)
+__device__ __forceinline__ void store_tf(double* base, const Reg& R, int f, const double* flx, double pg, double ug)
 {
     using T = TF<NS>;
-    base[f + R.np * T::RHO] = flx[URHO];
-    base[f + R.np * T::MX] = flx[UMX];
-    base[f + R.np * T::MY] = flx[UMY];
-    base[f + R.np * T::MZ] = flx[UMZ];
-    base[f + R.np * T::ED] = flx[UEDEN];
+    (base + f)[R.plane(T::RHO)] = flx[URHO];
+    (base + f)[R.plane(T::MX)] = flx[UMX];
+    (base + f)[R.plane(T::MY)] = flx[UMY];
+    (base + f)[R.plane(T::MZ)] = flx[UMZ];
+    (base + f)[R.plane(T::ED)] = flx[UEDEN];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) base[f + R.np * (T::X + n)] = flx[UFS + n];
-    base[f + R.np * T::PG] = pg;
-    base[f + R.np * T::UG] = ug;
+    for (int n = 0; n < NS; ++n) (base + f)[R.plane(T::X + n)] = flx[UFS + n];
+    (base + f)[R.plane(T::PG)] = pg;
+    (base + f)[R.plane(T::UG)] = ug;
 }
 
 template <int NS>
-__device__ __forceinline__ void load_tf(const double* base, const Reg& R, long long f, double* r)
+__device__ __forceinline__ void load_tf(const double* base, const Reg& R, int f, double* r)
 {
 #pragma unroll
-    for (int c = 0; c < TF<NS>::N; ++c) r[c] = base[f + R.np * c];
+    for (int c = 0; c < TF<NS>::N; ++c) r[c] = (base + f)[R.plane(c)];
 }
 
 // riemann1: compute_flux on tbx[d][d] (Castro_hydro.cpp:214-224)
@@ -677,10 +724,10 @@ __device__ __forceinline__ void riemann1_body(const SimDev& S, const Work& w)
     const BoxDev& B = S.boxes[b];
     constexpr int NQS = Dims<NS>::NQS, NVAR = Dims<NS>::NVAR;
     const double* T = S.Tr + B.offTr[d];
-    long long f = ridx(R, i, j, k);
+    const int f = ridx(R, i, j, k);
     double ql[NQS], qr[NQS];
 #pragma unroll
-    for (int c = 0; c < NQS; ++c) { ql[c] = T[f + R.np * c]; qr[c] = T[f + R.np * (NQS + c)]; }
+    for (int c = 0; c < NQS; ++c) { ql[c] = (T + f)[R.plane(c)]; qr[c] = (T + f)[R.plane(NQS + c)]; }
     QLoader<NS> ld;
     ld.base = S.Q + B.offQ;
     ld.R = q_region(S.inst[B.inst]);
@@ -760,17 +807,17 @@ __device__ __forceinline__ void cross_flux_store(const SimDev& S, const BoxDev& 
     riemann_cgf<NS, A>(st2[0], st2[1], gl, gr, cl, cr, flx, qg, nullptr);
     const Reg R = make_reg(B.lo, B.hi, R_TBX, 3 * A + Bd);
     double* out = S.F2 + B.offF2[pair_index(A, Bd)];
-    const long long f = ridx(R, i, j, k);
+    const int f = ridx(R, i, j, k);
     using T_ = TF<NS>;
-    out[f + R.np * T_::RHO] = flx[URHO];
-    out[f + R.np * T_::MX] = flx[UMX];
-    out[f + R.np * T_::MY] = flx[UMY];
-    out[f + R.np * T_::MZ] = flx[UMZ];
-    out[f + R.np * T_::ED] = flx[UEDEN];
+    (out + f)[R.plane(T_::RHO)] = flx[URHO];
+    (out + f)[R.plane(T_::MX)] = flx[UMX];
+    (out + f)[R.plane(T_::MY)] = flx[UMY];
+    (out + f)[R.plane(T_::MZ)] = flx[UMZ];
+    (out + f)[R.plane(T_::ED)] = flx[UEDEN];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) out[f + R.np * (T_::X + n)] = flx[UFS + n];
-    out[f + R.np * T_::PG] = qg[GDPRES];
-    out[f + R.np * T_::UG] = qg[GDU + A];
+    for (int n = 0; n < NS; ++n) (out + f)[R.plane(T_::X + n)] = flx[UFS + n];
+    (out + f)[R.plane(T_::PG)] = qg[GDPRES];
+    (out + f)[R.plane(T_::UG)] = qg[GDU + A];
 }
 
 // Both cross fluxes of the A-normal face (i,j,k) of tbx[A][A]: F^{A|B1} where
@@ -787,8 +834,8 @@ __device__ __forceinline__ void cross_flux_both(const SimDev& S, const BoxDev& B
     constexpr int eax = A == 0, eay = A == 1, eaz = A == 2;
     const Reg RT = make_reg(B.lo, B.hi, R_TBX, 4 * A);
     const double* T = S.Tr + B.offTr[A];
-    const long long ft = ridx(RT, i, j, k);
-    const long long zl = ridx(ld.R, i - eax, j - eay, k - eaz), zr = ridx(ld.R, i, j, k);
+    const int ft = ridx(RT, i, j, k);
+    const int zl = ridx(ld.R, i - eax, j - eay, k - eaz), zr = ridx(ld.R, i, j, k);
     double lqr[SL::ON ? 1 : 2 * NQS];
     const double* lq;
     double gl, gr;
@@ -796,21 +843,21 @@ __device__ __forceinline__ void cross_flux_both(const SimDev& S, const BoxDev& B
         extern __shared__ double r2_smem[];
         double* sm = r2_smem + threadIdx.x * SL::STRIDE;
 #pragma unroll
-        for (int c = 0; c < 2 * NQS; ++c) cp_async8(sm + SL::LQ + c, T + ft + RT.np * c);
-        cp_async8(sm + SL::G, ld.base + zl + ld.R.np * QF<NS>::GAMC);
-        cp_async8(sm + SL::G + 1, ld.base + zr + ld.R.np * QF<NS>::GAMC);
+        for (int c = 0; c < 2 * NQS; ++c) cp_async8(sm + SL::LQ + c, T + ft + RT.plane(c));
+        cp_async8(sm + SL::G, ld.base + zl + ld.R.plane(QF<NS>::GAMC));
+        cp_async8(sm + SL::G + 1, ld.base + zr + ld.R.plane(QF<NS>::GAMC));
         lq = sm + SL::LQ;
         cp_async_wait_all();
         gl = sm[SL::G];
         gr = sm[SL::G + 1];
     } else {
 #pragma unroll
-        for (int c = 0; c < 2 * NQS; ++c) lqr[c] = T[ft + RT.np * c];
+        for (int c = 0; c < 2 * NQS; ++c) lqr[c] = (T + ft)[RT.plane(c)];
         lq = lqr;
-        gl = ld.base[zl + ld.R.np * QF<NS>::GAMC];
-        gr = ld.base[zr + ld.R.np * QF<NS>::GAMC];
+        gl = (ld.base + zl)[ld.R.plane(QF<NS>::GAMC)];
+        gr = (ld.base + zr)[ld.R.plane(QF<NS>::GAMC)];
     }
-    const double cl = ld.base[zl + ld.R.np * QF<NS>::C], cr = ld.base[zr + ld.R.np * QF<NS>::C];
+    const double cl = (ld.base + zl)[ld.R.plane(QF<NS>::C)], cr = (ld.base + zr)[ld.R.plane(QF<NS>::C)];
     const int p[3] = {i, j, k};
     if (p[B1] >= B.lo[B1] && p[B1] <= B.hi[B1])
         cross_flux_store<NS, A, B1>(S, B, i, j, k, dt / I.dx[B1] / 3.0, lq, gl, gr, cl, cr);
@@ -902,25 +949,25 @@ __device__ __forceinline__ void final_flux(const SimDev& S, const BoxDev& B, con
     const double* T = S.Tr + B.offTr[D];
     const double* Dv = S.Div + B.offDiv;
     const double* Ub = S.Ub + B.offUb;
-    const long long ft = ridx(RT, i, j, k);
-    const long long c0 = ridx(RU, i, j, k), cm = ridx(RU, i - ex, j - ey, k - ez);
-    const long long zl = ridx(ld.R, i - ex, j - ey, k - ez), zr = ridx(ld.R, i, j, k);
+    const int ft = ridx(RT, i, j, k);
+    const int c0 = ridx(RU, i, j, k), cm = ridx(RU, i - ex, j - ey, k - ez);
+    const int zl = ridx(ld.R, i - ex, j - ey, k - ez), zr = ridx(ld.R, i, j, k);
     if constexpr (STG) {
 #pragma unroll
-        for (int c = 0; c < 2 * NQS; ++c) cp_async8(sm + SL::LQ + c, T + ft + RT.np * c);
-        cp_async8(sm + SL::G, ld.base + zl + ld.R.np * QF<NS>::GAMC);
-        cp_async8(sm + SL::G + 1, ld.base + zr + ld.R.np * QF<NS>::GAMC);
+        for (int c = 0; c < 2 * NQS; ++c) cp_async8(sm + SL::LQ + c, T + ft + RT.plane(c));
+        cp_async8(sm + SL::G, ld.base + zl + ld.R.plane(QF<NS>::GAMC));
+        cp_async8(sm + SL::G + 1, ld.base + zr + ld.R.plane(QF<NS>::GAMC));
 #pragma unroll
         for (int n = 0; n < NVAR; ++n) {
             if (n == UTEMP) continue;
-            cp_async8(sm + SL::UB + n, Ub + c0 + RU.np * n);
-            cp_async8(sm + SL::UB + NVAR + n, Ub + cm + RU.np * n);
+            cp_async8(sm + SL::UB + n, Ub + c0 + RU.plane(n));
+            cp_async8(sm + SL::UB + NVAR + n, Ub + cm + RU.plane(n));
         }
 #pragma unroll
         for (int m = 0; m < 4; ++m)
             cp_async8(sm + SL::DV + m, Dv + ridx(R1, i + AV_NODE[D][m][0], j + AV_NODE[D][m][1], k + AV_NODE[D][m][2]));
     }
-    const double cl = ld.base[zl + ld.R.np * QF<NS>::C], cr = ld.base[zr + ld.R.np * QF<NS>::C];
+    const double cl = (ld.base + zl)[ld.R.plane(QF<NS>::C)], cr = (ld.base + zr)[ld.R.plane(QF<NS>::C)];
     double st2[2][NQS];
 #pragma unroll
     for (int Dm = -1; Dm <= 0; ++Dm) {
@@ -928,7 +975,7 @@ __device__ __forceinline__ void final_flux(const SimDev& S, const BoxDev& B, con
         const int off = (Dm == -1) ? 0 : NQS;
         if constexpr (!STG) {
 #pragma unroll
-            for (int c = 0; c < NQS; ++c) lqr[c] = T[ft + RT.np * (off + c)];
+            for (int c = 0; c < NQS; ++c) lqr[c] = (T + ft)[RT.plane(off + c)];
         }
         int il = i + Dm * ex, jl = j + Dm * ey, kl = k + Dm * ez;
         f12(il + e1x, jl + e1y, kl + e1z, f2r);
@@ -961,8 +1008,8 @@ __device__ __forceinline__ void final_flux(const SimDev& S, const BoxDev& B, con
 #pragma unroll
         for (int n = 0; n < NVAR; ++n) {
             if (n == UTEMP) continue;
-            const double u0 = STG ? sm[SL::UB + n] : Ub[c0 + RU.np * n];
-            const double um = STG ? sm[SL::UB + NVAR + n] : Ub[cm + RU.np * n];
+            const double u0 = STG ? sm[SL::UB + n] : (Ub + c0)[RU.plane(n)];
+            const double um = STG ? sm[SL::UB + NVAR + n] : (Ub + cm)[RU.plane(n)];
             double div1 = av_term(ds, u0 - um);
             flx[n] = flx[n] + dxd * div1;
         }
@@ -979,14 +1026,14 @@ __device__ __forceinline__ void final_flux(const SimDev& S, const BoxDev& B, con
     // final record: every flux component but UTEMP (always zero), GDPRES, GDU_D
     Reg R = make_reg(B.lo, B.hi, R_EBX, D);
     double* X = S.Fx + B.offFx[D];
-    long long f = ridx(R, i, j, k);
+    const int f = ridx(R, i, j, k);
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) {
         if (n == UTEMP) continue;
-        X[f + R.np * (n < UTEMP ? n : n - 1)] = flx[n];
+        (X + f)[R.plane(n < UTEMP ? n : n - 1)] = flx[n];
     }
-    X[f + R.np * (NVAR - 1)] = g.x;
-    X[f + R.np * NVAR] = g.y;
+    (X + f)[R.plane(NVAR - 1)] = g.x;
+    (X + f)[R.plane(NVAR)] = g.y;
 }
 
 template <int NS>
@@ -1158,13 +1205,13 @@ __device__ __forceinline__ void cross_one(const SimDev& S, const BoxDev& B, cons
     constexpr int eax = A == 0, eay = A == 1, eaz = A == 2;
     const Reg RT = make_reg(B.lo, B.hi, R_TBX, 4 * A);
     const double* T = S.Tr + B.offTr[A];
-    const long long ft = ridx(RT, i, j, k);
+    const int ft = ridx(RT, i, j, k);
     double lq[2 * NQS];
 #pragma unroll
-    for (int c = 0; c < 2 * NQS; ++c) lq[c] = T[ft + RT.np * c];
-    const long long zl = ridx(ld.R, i - eax, j - eay, k - eaz), zr = ridx(ld.R, i, j, k);
-    const double gl = ld.base[zl + ld.R.np * QF<NS>::GAMC], gr = ld.base[zr + ld.R.np * QF<NS>::GAMC];
-    const double cl = ld.base[zl + ld.R.np * QF<NS>::C], cr = ld.base[zr + ld.R.np * QF<NS>::C];
+    for (int c = 0; c < 2 * NQS; ++c) lq[c] = (T + ft)[RT.plane(c)];
+    const int zl = ridx(ld.R, i - eax, j - eay, k - eaz), zr = ridx(ld.R, i, j, k);
+    const double gl = (ld.base + zl)[ld.R.plane(QF<NS>::GAMC)], gr = (ld.base + zr)[ld.R.plane(QF<NS>::GAMC)];
+    const double cl = (ld.base + zl)[ld.R.plane(QF<NS>::C)], cr = (ld.base + zr)[ld.R.plane(QF<NS>::C)];
     cross_flux_rec<NS, A, Bd>(S, B, i, j, k, dt / I.dx[Bd] / 3.0, lq, gl, gr, cl, cr, out, stride);
 }
 
@@ -1284,7 +1331,7 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
         const double volinv = 1.0 / (I.dx[0] * I.dx[1] * I.dx[2]);
         Reg RX[3];
         const double* X[3];
-        long long f0[3], f1[3];
+        int f0[3], f1[3];
         const BoxDev& DB = S.dom[B.inst];   // final fluxes live on the domain's faces
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -1294,24 +1341,24 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
             f1[d] = ridx(RX[d], i + (d == 0), j + (d == 1), k + (d == 2));
         }
         double* U = S.U + B.offU;
-        long long id = ridx(R, i, j, k);
+        const int id = ridx(R, i, j, k);
         double u[NVAR];
 #pragma unroll
         for (int n = 0; n < NVAR; ++n) {
-            double un = U[id + R.np * n];
+            double un = (U + id)[R.plane(n)];
             if (n == UTEMP) { u[n] = un + dt * 0.0; continue; }
             const int c = n < UTEMP ? n : n - 1;
-            double src = 0.0 + (X[0][f0[0] + RX[0].np * c] * a0 - X[0][f1[0] + RX[0].np * c] * a0
-                              + X[1][f0[1] + RX[1].np * c] * a1 - X[1][f1[1] + RX[1].np * c] * a1
-                              + X[2][f0[2] + RX[2].np * c] * a2 - X[2][f1[2] + RX[2].np * c] * a2) * volinv;
+            double src = 0.0 + ((X[0] + f0[0])[RX[0].plane(c)] * a0 - (X[0] + f1[0])[RX[0].plane(c)] * a0
+                              + (X[1] + f0[1])[RX[1].plane(c)] * a1 - (X[1] + f1[1])[RX[1].plane(c)] * a1
+                              + (X[2] + f0[2])[RX[2].plane(c)] * a2 - (X[2] + f1[2])[RX[2].plane(c)] * a2) * volinv;
             if (n == UEINT) {
                 const int P = NVAR - 1, V = NVAR;
-                double pdivu = 0.5 * (X[0][f1[0] + RX[0].np * P] + X[0][f0[0] + RX[0].np * P]) *
-                                   (X[0][f1[0] + RX[0].np * V] - X[0][f0[0] + RX[0].np * V]) / I.dx[0] +
-                               0.5 * (X[1][f1[1] + RX[1].np * P] + X[1][f0[1] + RX[1].np * P]) *
-                                   (X[1][f1[1] + RX[1].np * V] - X[1][f0[1] + RX[1].np * V]) / I.dx[1] +
-                               0.5 * (X[2][f1[2] + RX[2].np * P] + X[2][f0[2] + RX[2].np * P]) *
-                                   (X[2][f1[2] + RX[2].np * V] - X[2][f0[2] + RX[2].np * V]) / I.dx[2];
+                double pdivu = 0.5 * ((X[0] + f1[0])[RX[0].plane(P)] + (X[0] + f0[0])[RX[0].plane(P)]) *
+                                   ((X[0] + f1[0])[RX[0].plane(V)] - (X[0] + f0[0])[RX[0].plane(V)]) / I.dx[0] +
+                               0.5 * ((X[1] + f1[1])[RX[1].plane(P)] + (X[1] + f0[1])[RX[1].plane(P)]) *
+                                   ((X[1] + f1[1])[RX[1].plane(V)] - (X[1] + f0[1])[RX[1].plane(V)]) / I.dx[1] +
+                               0.5 * ((X[2] + f1[2])[RX[2].plane(P)] + (X[2] + f0[2])[RX[2].plane(P)]) *
+                                   ((X[2] + f1[2])[RX[2].plane(V)] - (X[2] + f0[2])[RX[2].plane(V)]) / I.dx[2];
                 src = src - pdivu;
             }
             u[n] = un + dt * src;                        // MultiFab::Saxpy, Castro_advance.cpp:74
@@ -1319,7 +1366,7 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
         clean_state_pt<NS, COUL>(u);                     // Castro_advance.cpp:78
         clean_state_pt<NS, COUL>(u);                     // Castro.cpp:369
 #pragma unroll
-        for (int n = 0; n < NVAR; ++n) U[id + R.np * n] = u[n];
+        for (int n = 0; n < NVAR; ++n) (U + id)[R.plane(n)] = u[n];
         m = estdt_pt<NS, COUL>(u, I.dx[0], I.dx[1], I.dx[2]);   // Castro.cpp:191-203 of the next coarse step
     }
     // one box per block: the block reduction has a single instance target
@@ -1346,10 +1393,10 @@ __device__ __forceinline__ void estdt_state_body(const SimDev& S, const Work& w)
     if (active) {
         constexpr int NVAR = Dims<NS>::NVAR;
         const double* U = S.U + B.offU;
-        long long id = ridx(R, i, j, k);
+        const int id = ridx(R, i, j, k);
         double u[NVAR];
 #pragma unroll
-        for (int n = 0; n < NVAR; ++n) u[n] = U[id + R.np * n];
+        for (int n = 0; n < NVAR; ++n) u[n] = (U + id)[R.plane(n)];
         m = estdt_pt<NS, COUL>(u, I.dx[0], I.dx[1], I.dx[2]);
     }
     m = block_min(m);
@@ -1552,9 +1599,9 @@ __global__ void __launch_bounds__(BLOCK) k_fill_sborder(SimDev S, int b, double*
     const BoxDev& O = S.boxes[ob];
     Reg RO = make_reg(O.lo, O.hi, R_VALID, 0);
     const double* Us = S.U + O.offU;
-    long long is = ridx(RO, ii, jj, kk);
+    const int is = ridx(RO, ii, jj, kk);
 #pragma unroll
-    for (int n = 0; n < Dims<NS>::NVAR; ++n) sb[t + R.np * n] = Us[is + RO.np * n];
+    for (int n = 0; n < Dims<NS>::NVAR; ++n) (sb + t)[R.plane(n)] = (Us + is)[RO.plane(n)];
 }
 
 // primitive variables straight from a caller's Sborder over grow(bx,4)
@@ -1575,24 +1622,24 @@ __global__ void __launch_bounds__(BLOCK) k_box_prim(SimDev S, const Work* wl, Fa
     const InstDev& I = S.inst[B.inst];
     const Reg RQ = q_region(I);   // grow(bx,4): the instance domain is the box here
     double* Q = S.Q + B.offQ;
-    long long id = ridx(RQ, i, j, k);
+    const int id = ridx(RQ, i, j, k);
     using F = QF<NS>;
-    Q[id + RQ.np * F::RHO] = q[QRHO];
-    Q[id + RQ.np * (F::U + 0)] = q[QU];
-    Q[id + RQ.np * (F::U + 1)] = q[QV];
-    Q[id + RQ.np * (F::U + 2)] = q[QW];
-    Q[id + RQ.np * F::P] = q[QPRES];
-    Q[id + RQ.np * F::RE] = q[QREINT];
+    (Q + id)[RQ.plane(F::RHO)] = q[QRHO];
+    (Q + id)[RQ.plane(F::U + 0)] = q[QU];
+    (Q + id)[RQ.plane(F::U + 1)] = q[QV];
+    (Q + id)[RQ.plane(F::U + 2)] = q[QW];
+    (Q + id)[RQ.plane(F::P)] = q[QPRES];
+    (Q + id)[RQ.plane(F::RE)] = q[QREINT];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) Q[id + RQ.np * (F::X + n)] = q[QFS + n];
-    Q[id + RQ.np * F::GAMC] = qa[QGAMC];
-    Q[id + RQ.np * F::C] = qa[QC];
+    for (int n = 0; n < NS; ++n) (Q + id)[RQ.plane(F::X + n)] = q[QFS + n];
+    (Q + id)[RQ.plane(F::GAMC)] = qa[QGAMC];
+    (Q + id)[RQ.plane(F::C)] = qa[QC];
     if (i >= B.lo[0] - 1 && i <= B.hi[0] + 1 && j >= B.lo[1] - 1 && j <= B.hi[1] + 1 && k >= B.lo[2] - 1 && k <= B.hi[2] + 1) {
         const Reg R1 = u_region(I);
         double* Ub = S.Ub + B.offUb;
-        long long i1 = ridx(R1, i, j, k);
+        const int i1 = ridx(R1, i, j, k);
 #pragma unroll
-        for (int n = 0; n < NVAR; ++n) Ub[i1 + R1.np * n] = u[n];
+        for (int n = 0; n < NVAR; ++n) (Ub + i1)[R1.plane(n)] = u[n];
     }
 }
 
@@ -1611,7 +1658,7 @@ __global__ void __launch_bounds__(BLOCK) k_box_source(SimDev S, const Work* wl, 
     const double volinv = 1.0 / (I.dx[0] * I.dx[1] * I.dx[2]);
     Reg RX[3];
     const double* X[3];
-    long long f0[3], f1[3];
+    int f0[3], f1[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         RX[d] = make_reg(B.lo, B.hi, R_EBX, d);
@@ -1623,17 +1670,17 @@ __global__ void __launch_bounds__(BLOCK) k_box_source(SimDev S, const Work* wl, 
     for (int n = 0; n < NVAR; ++n) {
         if (n == UTEMP) { SRC(i, j, k, n) = SRC(i, j, k, n) + 0.0 * volinv; continue; }
         const int c = n < UTEMP ? n : n - 1;
-        double s = SRC(i, j, k, n) + (X[0][f0[0] + RX[0].np * c] * a0 - X[0][f1[0] + RX[0].np * c] * a0
-                                    + X[1][f0[1] + RX[1].np * c] * a1 - X[1][f1[1] + RX[1].np * c] * a1
-                                    + X[2][f0[2] + RX[2].np * c] * a2 - X[2][f1[2] + RX[2].np * c] * a2) * volinv;
+        double s = SRC(i, j, k, n) + ((X[0] + f0[0])[RX[0].plane(c)] * a0 - (X[0] + f1[0])[RX[0].plane(c)] * a0
+                                    + (X[1] + f0[1])[RX[1].plane(c)] * a1 - (X[1] + f1[1])[RX[1].plane(c)] * a1
+                                    + (X[2] + f0[2])[RX[2].plane(c)] * a2 - (X[2] + f1[2])[RX[2].plane(c)] * a2) * volinv;
         if (n == UEINT) {
             const int P = NVAR - 1, V = NVAR;
-            double pdivu = 0.5 * (X[0][f1[0] + RX[0].np * P] + X[0][f0[0] + RX[0].np * P]) *
-                               (X[0][f1[0] + RX[0].np * V] - X[0][f0[0] + RX[0].np * V]) / I.dx[0] +
-                           0.5 * (X[1][f1[1] + RX[1].np * P] + X[1][f0[1] + RX[1].np * P]) *
-                               (X[1][f1[1] + RX[1].np * V] - X[1][f0[1] + RX[1].np * V]) / I.dx[1] +
-                           0.5 * (X[2][f1[2] + RX[2].np * P] + X[2][f0[2] + RX[2].np * P]) *
-                               (X[2][f1[2] + RX[2].np * V] - X[2][f0[2] + RX[2].np * V]) / I.dx[2];
+            double pdivu = 0.5 * ((X[0] + f1[0])[RX[0].plane(P)] + (X[0] + f0[0])[RX[0].plane(P)]) *
+                               ((X[0] + f1[0])[RX[0].plane(V)] - (X[0] + f0[0])[RX[0].plane(V)]) / I.dx[0] +
+                           0.5 * ((X[1] + f1[1])[RX[1].plane(P)] + (X[1] + f0[1])[RX[1].plane(P)]) *
+                               ((X[1] + f1[1])[RX[1].plane(V)] - (X[1] + f0[1])[RX[1].plane(V)]) / I.dx[1] +
+                           0.5 * ((X[2] + f1[2])[RX[2].plane(P)] + (X[2] + f0[2])[RX[2].plane(P)]) *
+                               ((X[2] + f1[2])[RX[2].plane(V)] - (X[2] + f0[2])[RX[2].plane(V)]) / I.dx[2];
             s = s - pdivu;
         }
         SRC(i, j, k, n) = s;
@@ -1654,10 +1701,10 @@ __global__ void __launch_bounds__(BLOCK) k_box_store_flux(SimDev S, const Work* 
     if (!FO.p) return;
     const double area = d == 0 ? I.dx[1] * I.dx[2] : d == 1 ? I.dx[0] * I.dx[2] : I.dx[0] * I.dx[1];
     const double* X = S.Fx + B.offFx[d];
-    long long f = ridx(R, i, j, k);
+    const int f = ridx(R, i, j, k);
 #pragma unroll
     for (int n = 0; n < Dims<NS>::NVAR; ++n) {
-        double F = (n == UTEMP) ? 0.0 : X[f + R.np * (n < UTEMP ? n : n - 1)];
+        double F = (n == UTEMP) ? 0.0 : (X + f)[R.plane(n < UTEMP ? n : n - 1)];
         FO(i, j, k, n) = dt * F * area;
     }
 }
@@ -1708,9 +1755,9 @@ struct castro_sim {
     double *Tr = nullptr, *F1 = nullptr, *F2 = nullptr, *Fx = nullptr;
     long long nU = 0;
     // work lists
-    Work *w_valid = nullptr, *w_g4 = nullptr, *w_g1 = nullptr, *w_trace = nullptr, *w_tbx = nullptr,
-         *w_ebx = nullptr, *w_r2 = nullptr, *w_r3 = nullptr, *w_ghost = nullptr;
-    int n_valid = 0, n_g4 = 0, n_g1 = 0, n_trace = 0, n_tbx = 0, n_ebx = 0, n_r2 = 0, n_r3 = 0, n_ghost = 0;
+    Work *w_valid = nullptr, *w_g1 = nullptr, *w_trace = nullptr, *w_tbx = nullptr, *w_r2 = nullptr, *w_r3 = nullptr,
+         *w_ghost = nullptr;
+    int n_valid = 0, n_g1 = 0, n_trace = 0, n_tbx = 0, n_r2 = 0, n_r3 = 0, n_ghost = 0;
     // column tiles of riemann23 (2 species, batched mode): the step runs it in place of riemann2 + riemann3
     TileItem* w_r23 = nullptr;
     int n_r23 = 0;
@@ -1771,8 +1818,8 @@ namespace {
 
 long long npts_reg(const int* lo, const int* hi, int kind, int sub)
 {
-    Reg r = make_reg(lo, hi, kind, sub);
-    return r.np;
+    const Reg r = make_reg(lo, hi, kind, sub);
+    return (long long)r.nx * r.ny * r.nz;
 }
 
 bool cuda_ok(cudaError_t e, const char* what)
@@ -1805,19 +1852,10 @@ void build_work(const std::vector<BoxDev>& boxes, int kind, int nsub, int tbx_mo
             int rs = sub;
             if (kind == R_TBX && tbx_mode == 0) rs = 4 * sub;
             long long np = npts_reg(B.lo, B.hi, kind, rs);
-            if (np > 2147483647LL - BLOCK) {   // work items carry 32-bit offsets
-                set_error(CASTRO_ERR_ARG, "castro_sim_create: a domain region exceeds 2^31 points");
-                *count = 0;
-                return;
-            }
+            const Reg R = make_reg(B.lo, B.hi, kind, rs);
             const long long chunk = (long long)BLOCK * passes;
             for (long long st = 0; st < np; st += chunk) {
-                Work it;
-                it.box = (int)b;
-                it.sub = sub;
-                it.start = (int)st;
-                it.count = (int)std::min<long long>(chunk, np - st);
-                w.push_back(it);
+                w.push_back(make_work((int)b, sub, st, (int)std::min<long long>(chunk, np - st), R));
             }
         }
     }
@@ -1851,14 +1889,9 @@ void build_ghost_work(castro_sim* s)
         for (int in = 0; in < s->ninst; ++in) {
             const InstDev& I = s->hinst[in];
             const long long np = npts_reg(I.dom_lo, I.dom_hi, R_GHOST, sub);
-            for (long long st = 0; st < np; st += BLOCK) {
-                Work it;
-                it.box = s->inst_boxes[in][0];
-                it.sub = sub;
-                it.start = (int)st;
-                it.count = (int)std::min<long long>(BLOCK, np - st);
-                w.push_back(it);
-            }
+            const Reg R = make_reg(I.dom_lo, I.dom_hi, R_GHOST, sub);
+            for (long long st = 0; st < np; st += BLOCK)
+                w.push_back(make_work(s->inst_boxes[in][0], sub, st, (int)std::min<long long>(BLOCK, np - st), R));
         }
     s->n_ghost = (int)w.size();
     if (dalloc(&s->w_ghost, w.size(), "ghost work list"))
@@ -2492,6 +2525,11 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
         for (int a = 0; a < 3; ++a)
             for (int bb = 0; bb < 3; ++bb)
                 if (a != bb) { P.offF2[pair_index(a, bb)] = oF2; oF2 += npts_reg(P.lo, P.hi, R_TBX, 3 * a + bb) * NTF; }
+        if (npts_reg(P.lo, P.hi, R_G4, 0) > 2147483647LL - MAX_ITEM) {   // the largest region
+            set_error(CASTRO_ERR_ARG, "castro_sim_create: a domain region exceeds 2^31 points");
+            castro_sim_destroy(s);
+            return nullptr;
+        }
         size_t nown = (size_t)I.on[0] * I.on[1] * I.on[2];
         owner_all.resize(owner_all.size() + nown, -1);
         for (int b = 0; b < D.nbox; ++b) {
@@ -2551,12 +2589,10 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
         ok = dalloc(&s->Ub, oUb, "Ub") && dalloc(&s->Q, oQ, "Q") && dalloc(&s->Div, oDiv, "Div") &&
              dalloc(&s->Tr, oTr, "Tr") && dalloc(&s->F1, oF1, "F1") && dalloc(&s->F2, oF2, "F2") && dalloc(&s->Fx, oFx, "Fx");
         build_work(s->hboxes, R_VALID, 1, -1, &s->w_valid, &s->n_valid);
-        build_work(s->hboxes, R_G4, 1, -1, &s->w_g4, &s->n_g4);
         // the stage kernels walk the domain boxes (launched with dev_dom())
         build_work(s->hdom, R_G1, 1, -1, &s->w_g1, &s->n_g1);
         build_work(s->hdom, R_SEG, 3, -1, &s->w_trace, &s->n_trace);
         build_work(s->hdom, R_TBX, 3, 0, &s->w_tbx, &s->n_tbx);
-        build_work(s->hdom, R_EBX, 3, -1, &s->w_ebx, &s->n_ebx);
         build_work(s->hdom, R_TBX, 3, 0, &s->w_r2, &s->n_r2, CASTRO_R2_ROWS);
         build_work(s->hdom, R_EBX, 3, -1, &s->w_r3, &s->n_r3, CASTRO_R3_ROWS);
         build_ghost_work(s);
@@ -2599,7 +2635,7 @@ void castro_sim_destroy(castro_sim* s)
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
     if (s->graph) cudaGraphDestroy(s->graph);
     void* ptrs[] = {s->dboxes, s->ddom, s->dinst, s->dstate, s->downer, s->U, s->Ub, s->Q, s->Div, s->Tr, s->F1, s->F2, s->Fx,
-                    s->w_valid, s->w_g4, s->w_g1, s->w_trace, s->w_tbx, s->w_ebx, s->w_r2, s->w_r3, s->w_ghost, s->sb, s->src,
+                    s->w_valid, s->w_g1, s->w_trace, s->w_tbx, s->w_r2, s->w_r3, s->w_ghost, s->sb, s->src,
                     s->d_dtloc, s->d_dtbox, s->pctl, s->w_r23};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -3109,12 +3145,10 @@ __global__ void k_noalloc_setup(BoxDev B, InstDev I, InstState st, NoallocLists 
         long long np = NLs.np[l][sub];
         int nb = (int)((np + BLOCK - 1) / BLOCK);
         if (item < nb) {
-            Work w;
-            w.box = 0;
-            w.sub = sub;
-            w.start = item * BLOCK;
-            w.count = (int)(np - (long long)item * BLOCK < BLOCK ? np - (long long)item * BLOCK : BLOCK);
-            work[t] = w;
+            const long long st = (long long)item * BLOCK;
+            const int kinds[NL_COUNT] = {R_VALID, R_G4, R_G1, R_SEG, R_TBX, R_EBX};
+            work[t] = make_work(0, sub, st, (int)(np - st < BLOCK ? np - st : BLOCK),
+                                make_reg(B.lo, B.hi, kinds[l], l == NL_TBX ? 4 * sub : sub));
             return;
         }
         item -= nb;

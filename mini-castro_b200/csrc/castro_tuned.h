@@ -38,7 +38,7 @@
 #define CASTRO_MINB_EOS 4
 #endif
 #ifndef CASTRO_MINB_R3
-#define CASTRO_MINB_R3 0
+#define CASTRO_MINB_R3 4
 #endif
 #ifndef CASTRO_MINB_RIEMANN
 #define CASTRO_MINB_RIEMANN 5
