@@ -41,9 +41,9 @@ import build as B  # noqa: E402
 KNOBS = [
     ("CASTRO_BLOCK", [64, 128, 256]),
     ("CASTRO_MINB_EOS", [0, 2, 3, 4]),
-    ("CASTRO_MINB_R3", [0, 2, 3, 4]),
+    ("CASTRO_MINB_R3", [0, 3, 4, 5, 6]),
     ("CASTRO_MINB_TRACE", [0, 2, 3, 4]),
-    ("CASTRO_MINB_RIEMANN", [0, 3, 4, 5, 6]),
+    ("CASTRO_MINB_RIEMANN", [0, 4, 5, 6, 7, 8]),
     ("CASTRO_TRACE_SEG", [3, 5, 7, 9]),
     ("CASTRO_TRACE_SPLIT", [0, 1]),
     ("CASTRO_MINB_TRACE2", [0, 6, 8]),
@@ -52,9 +52,9 @@ KNOBS = [
     ("CASTRO_R2_ROWS", [1, 2, 4]),
     ("CASTRO_R3_ROWS", [1, 2, 4]),
 ]
-DEFAULTS = {"CASTRO_BLOCK": 128, "CASTRO_MINB_EOS": 4, "CASTRO_MINB_R3": 0, "CASTRO_MINB_TRACE": 3,
-            "CASTRO_MINB_RIEMANN": 5, "CASTRO_TRACE_SEG": 5, "CASTRO_R2_STAGE": 1, "CASTRO_R3_STAGE": 1,
-            "CASTRO_R2_ROWS": 1, "CASTRO_R3_ROWS": 2,
+DEFAULTS = {"CASTRO_BLOCK": 128, "CASTRO_MINB_EOS": 4, "CASTRO_MINB_R3": 4, "CASTRO_MINB_TRACE": 3,
+            "CASTRO_MINB_RIEMANN": 7, "CASTRO_TRACE_SEG": 5, "CASTRO_R2_STAGE": 1, "CASTRO_R3_STAGE": 0,
+            "CASTRO_R2_ROWS": 1, "CASTRO_R3_ROWS": 1,
             "CASTRO_TRACE_SPLIT": 1, "CASTRO_MINB_TRACE2": 0}
 
 

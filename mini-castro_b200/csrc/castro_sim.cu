@@ -76,13 +76,13 @@ constexpr int NG = 4;   // ghost zones of Sborder, Source/Castro_advance.cpp:37
 #define CASTRO_MINB_EOS 4
 #endif
 #ifndef CASTRO_MINB_R3
-#define CASTRO_MINB_R3 0
+#define CASTRO_MINB_R3 4
 #endif
 #ifndef CASTRO_MINB_TRACE
 #define CASTRO_MINB_TRACE 3
 #endif
 #ifndef CASTRO_MINB_RIEMANN
-#define CASTRO_MINB_RIEMANN 5
+#define CASTRO_MINB_RIEMANN 7
 #endif
 #ifndef CASTRO_TRACE_SEG
 #define CASTRO_TRACE_SEG 5
@@ -90,13 +90,12 @@ constexpr int NG = 4;   // ghost zones of Sborder, Source/Castro_advance.cpp:37
 constexpr int BLOCK = CASTRO_BLOCK;
 constexpr int TSEG = CASTRO_TRACE_SEG;   // zones of grow(bx,1) one trace thread walks along its direction
 // Passes of BLOCK consecutive faces one block of riemann2 / riemann3 makes in
-// turn on the batched path: the next pass's faces are the next row, whose
-// flux records the previous pass has brought into this SM's L1
+// turn on the batched path (1: measured best with the items in slabs of z)
 #ifndef CASTRO_R2_ROWS
 #define CASTRO_R2_ROWS 1
 #endif
 #ifndef CASTRO_R3_ROWS
-#define CASTRO_R3_ROWS 2
+#define CASTRO_R3_ROWS 1
 #endif
 // The 13-species instantiations carry larger records and take their own
 // register budgets (CASTRO_MINB13_*, 0 = the compiler's choice; measured on the
@@ -895,7 +894,8 @@ __global__ void LB_RIEMANN k_riemann2(SimDev S, const Work* wl)
 // neighbouring thread reads (both trace states, gamma_1, the two zones'
 // Sborder values and the four divu nodes of apply_av) staged in shared memory
 // by cp.async; the cross-flux records stay plain loads served from L1
-// (measured on B200: 0 is faster, 0.85 against 0.90 ms for the 128^3 step).
+// (measured on B200, 128^3, 2 species: 0 is faster, 637 against 657 us: the
+// 42 KB a block stages are taken from the L1 that serves the records).
 #ifndef CASTRO_R3_STAGE
 #define CASTRO_R3_STAGE 0
 #endif
@@ -1843,19 +1843,62 @@ bool dalloc(T** p, size_t n, const char* what)
 void build_work(const std::vector<BoxDev>& boxes, int kind, int nsub, int tbx_mode, Work** out, int* count,
                 int passes = 1)
 {
-    // sub-major order: every box's items of one direction before the next, so
-    // the blocks resident on an SM run the same code path
+    // Items in slabs of z: every direction's items of one slab before the next
+    // slab's, so that what the directions share -- Q for trace, the normal-flux
+    // records for riemann2 (each read by two directions' faces), Sborder and divu
+    // for riemann3 -- comes from DRAM once and from L2 after that.  A slab holds
+    // about 64 K zones (~70 MB of riemann2's and riemann3's operands, of 126 MB
+    // L2); with whole directions one after the other, 128^3 step, 2 species, B200:
+    // trace2 225 us (now 194), riemann2 654 (604), riemann3 675 (636).
+    constexpr long long SLAB_ZONES = 65536;
+    struct Walk {
+        Reg R;
+        long long st, np;
+        int zones;          // z zones per point of R (trace's segments)
+        Work next;
+    };
     std::vector<Work> w;
-    for (int sub = 0; sub < nsub; ++sub) {
-        for (size_t b = 0; b < boxes.size(); ++b) {
-            const BoxDev& B = boxes[b];
-            int rs = sub;
-            if (kind == R_TBX && tbx_mode == 0) rs = 4 * sub;
-            long long np = npts_reg(B.lo, B.hi, kind, rs);
-            const Reg R = make_reg(B.lo, B.hi, kind, rs);
-            const long long chunk = (long long)BLOCK * passes;
-            for (long long st = 0; st < np; st += chunk) {
-                w.push_back(make_work((int)b, sub, st, (int)std::min<long long>(chunk, np - st), R));
+    const long long chunk = (long long)BLOCK * passes;
+    auto region = [&](const BoxDev& B, int sub) {
+        return make_reg(B.lo, B.hi, kind, kind == R_TBX && tbx_mode == 0 ? 4 * sub : sub);
+    };
+    long long total = 0;
+    for (const BoxDev& B : boxes)
+        for (int sub = 0; sub < nsub; ++sub) {
+            const Reg R = region(B, sub);
+            total += ((long long)R.nx * R.ny * R.nz + chunk - 1) / chunk;
+        }
+    w.reserve((size_t)total);
+    for (size_t b = 0; b < boxes.size(); ++b) {
+        const BoxDev& B = boxes[b];
+        const long long plane = npts_reg(B.lo, B.hi, R_VALID, 0) / (B.hi[2] - B.lo[2] + 1);
+        const int height = (int)std::max<long long>(1, SLAB_ZONES / plane);
+        Walk walk[3];
+        bool more = false;
+        for (int sub = 0; sub < nsub; ++sub) {
+            Walk& q = walk[sub];
+            q.R = region(B, sub);
+            q.np = (long long)q.R.nx * q.R.ny * q.R.nz;
+            q.zones = (B.hi[2] - B.lo[2] + q.R.nz) / q.R.nz;
+            q.st = 0;
+            q.next = make_work((int)b, sub, 0, (int)std::min(chunk, q.np), q.R);
+            more = more || q.np > 0;
+        }
+        for (int slab = 0; more; ++slab) {
+            more = false;
+            for (int sub = 0; sub < nsub; ++sub) {
+                Walk& q = walk[sub];
+                while (q.st < q.np && q.next.k0 * q.zones < (slab + 1) * height) {
+                    w.push_back(q.next);
+                    q.st += chunk;
+                    // the next item's first point, carried over the row and the plane
+                    q.next.count = (int)std::min(chunk, q.np - q.st);
+                    const unsigned x = (unsigned)q.next.i0 + (unsigned)chunk, y = (unsigned)q.next.j0 + x / (unsigned)q.R.nx;
+                    q.next.i0 = (int)(x % (unsigned)q.R.nx);
+                    q.next.j0 = (int)(y % (unsigned)q.R.ny);
+                    q.next.k0 += (int)(y / (unsigned)q.R.ny);
+                }
+                more = more || q.st < q.np;
             }
         }
     }
@@ -2593,7 +2636,12 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
         build_work(s->hdom, R_G1, 1, -1, &s->w_g1, &s->n_g1);
         build_work(s->hdom, R_SEG, 3, -1, &s->w_trace, &s->n_trace);
         build_work(s->hdom, R_TBX, 3, 0, &s->w_tbx, &s->n_tbx);
-        build_work(s->hdom, R_TBX, 3, 0, &s->w_r2, &s->n_r2, CASTRO_R2_ROWS);
+        if (CASTRO_R2_ROWS == 1) {   // riemann1's items are riemann2's
+            s->w_r2 = s->w_tbx;
+            s->n_r2 = s->n_tbx;
+        } else {
+            build_work(s->hdom, R_TBX, 3, 0, &s->w_r2, &s->n_r2, CASTRO_R2_ROWS);
+        }
         build_work(s->hdom, R_EBX, 3, -1, &s->w_r3, &s->n_r3, CASTRO_R3_ROWS);
         build_ghost_work(s);
         if (ok && ns == 2 && column_tiles_on() && mode == CASTRO_MODE_BATCHED) ok = build_r23_work(s);
@@ -2635,7 +2683,7 @@ void castro_sim_destroy(castro_sim* s)
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
     if (s->graph) cudaGraphDestroy(s->graph);
     void* ptrs[] = {s->dboxes, s->ddom, s->dinst, s->dstate, s->downer, s->U, s->Ub, s->Q, s->Div, s->Tr, s->F1, s->F2, s->Fx,
-                    s->w_valid, s->w_g1, s->w_trace, s->w_tbx, s->w_r2, s->w_r3, s->w_ghost, s->sb, s->src,
+                    s->w_valid, s->w_g1, s->w_trace, s->w_tbx, CASTRO_R2_ROWS == 1 ? nullptr : s->w_r2, s->w_r3, s->w_ghost, s->sb, s->src,
                     s->d_dtloc, s->d_dtbox, s->pctl, s->w_r23};
     for (void* p : ptrs)
         if (p) cudaFree(p);

@@ -1,6 +1,11 @@
 // castro_tuned.h -- launch shape of the fused batched step, chosen by
 // mini-castro_b200/autotune.py from timings of the batched step
-// (sedov128_pert) on the GPU it ran on.  Timing table (ms per step):
+// (sedov128_pert) on the GPU it ran on, and by later sweeps of the Riemann
+// kernels on B200, which took the rows of riemann3, its staging and the blocks
+// per SM after the table: with 32-bit indices riemann1 / riemann2 fit seven
+// blocks (72 registers; 604 -> 566 us for riemann2 against five), and riemann3
+// without staging, one pass of faces per block and four blocks 637 us against
+// 657 staged with two passes.  Timing table of the autotuner (ms per step):
 //   block128_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    3.488
 //   block64_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    4.077
 //   block256_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    4.852
@@ -41,7 +46,7 @@
 #define CASTRO_MINB_R3 4
 #endif
 #ifndef CASTRO_MINB_RIEMANN
-#define CASTRO_MINB_RIEMANN 5
+#define CASTRO_MINB_RIEMANN 7
 #endif
 #ifndef CASTRO_MINB_TRACE
 #define CASTRO_MINB_TRACE 3
@@ -56,10 +61,10 @@
 #define CASTRO_R2_STAGE 1
 #endif
 #ifndef CASTRO_R3_ROWS
-#define CASTRO_R3_ROWS 2
+#define CASTRO_R3_ROWS 1
 #endif
 #ifndef CASTRO_R3_STAGE
-#define CASTRO_R3_STAGE 1
+#define CASTRO_R3_STAGE 0
 #endif
 #ifndef CASTRO_TRACE_SEG
 #define CASTRO_TRACE_SEG 5
