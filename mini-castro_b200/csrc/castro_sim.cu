@@ -366,10 +366,11 @@ __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
     const int id = ridx(R, i, j, k);
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) u[n] = (U + id)[R.plane(n)];
-    clean_state_pt<NS, COUL>(u);                    // Castro_advance.cpp:51
+    EosKnown known;
+    clean_state_pt<NS, COUL>(u, &known);            // Castro_advance.cpp:51
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) (U + id)[R.plane(n)] = u[n];
-    clean_state_pt<NS, COUL>(u);                    // Castro_advance.cpp:66 (valid part of Sborder)
+    clean_state_pt<NS, COUL>(u, &known);            // Castro_advance.cpp:66 (valid part of Sborder)
     const InstDev& I = S.inst[B.inst];
     const Reg R1 = u_region(I);
     double* Ub = S.Ub + B.offUb;
@@ -377,7 +378,7 @@ __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) (Ub + id1)[R1.plane(n)] = u[n];
     double q[QVAR], qa[NQAUX];
-    ctoprim_pt<NS, COUL>(u, q, qa);                 // Castro_hydro.cpp:64-70
+    ctoprim_pt<NS, COUL>(u, q, qa, &known);         // Castro_hydro.cpp:64-70
     const Reg R4 = q_region(I);
     double* Q = S.Q + B.offQ;
     const int id4 = ridx(R4, i, j, k);
@@ -1363,11 +1364,12 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
             }
             u[n] = un + dt * src;                        // MultiFab::Saxpy, Castro_advance.cpp:74
         }
-        clean_state_pt<NS, COUL>(u);                     // Castro_advance.cpp:78
-        clean_state_pt<NS, COUL>(u);                     // Castro.cpp:369
+        EosKnown known;
+        clean_state_pt<NS, COUL>(u, &known);             // Castro_advance.cpp:78
+        clean_state_pt<NS, COUL>(u, &known);             // Castro.cpp:369
 #pragma unroll
         for (int n = 0; n < NVAR; ++n) (U + id)[R.plane(n)] = u[n];
-        m = estdt_pt<NS, COUL>(u, I.dx[0], I.dx[1], I.dx[2]);   // Castro.cpp:191-203 of the next coarse step
+        m = estdt_pt<NS, COUL>(u, I.dx[0], I.dx[1], I.dx[2], &known);   // Castro.cpp:191-203 of the next coarse step
     }
     // one box per block: the block reduction has a single instance target
     m = block_min(m);
