@@ -975,6 +975,59 @@ CASTRO_HD void ppm_int_wave(double sm, double sp, double s6, double speed, doubl
     }
 }
 
+// van Leer slope (vl_slope) from the doubled left difference 2 (s0 - sm1),
+// which is the doubled right difference of the zone to the left: a walk along
+// zones forms each difference once and hands it on
+CASTRO_HD double vl_slope_walk(double sm1, double s0, double sp1, double& dsl)
+{
+    const double dsr = 2.0 * (sp1 - s0), dl = dsl;
+    dsl = dsr;
+    if (dl * dsr > 0.0) {
+        const double dsc = 0.5 * (sp1 - sm1);
+        return copysign(DMIN(DMIN(fabs(dsc), fabs(dl)), fabs(dsr)), dsc);
+    }
+    return 0.0;
+}
+
+// ppm_int_wave in one expression: for a wave to the left (speed <= 0) the
+// integral is Im and Ip is the plus edge, for one to the right it is Ip and Im
+// is the minus edge.  sp - h (d - k s6) = sp + h (-d + k s6) to the bit.
+struct Wave {
+    double h, k;     // sigma / 2, 1 - 2/3 sigma
+    bool left;
+    CASTRO_HD void set(double speed, double dtdx)
+    {
+        const double sigma = fabs(speed) * dtdx;
+        left = speed <= 0.0;
+        h = 0.5 * sigma;
+        k = 1.0 - TWO3RD * sigma;
+    }
+    CASTRO_HD double integral(double sm, double sp, double s6) const
+    {
+        const double d = sp - sm;
+        return (left ? sm : sp) + h * ((left ? d : -d) + k * s6);
+    }
+};
+
+CASTRO_HD void trace_project(const double I[3][4], double gam_g_ref, double un, double cc, bool plus, double& rho_o,
+                             double& un_o, double& rhoe_o, double& p_o);
+
+// One side's characteristic projection when it is not the usual case of
+// trace_states: trace_project with the integrals of the waves it reads
+CASTRO_HD void trace_side(double rho_i, double un_i, double p_i, double re_i, double rho1, double p1, double re1, double uo,
+                          double po, double gam, double un, double cc, bool plus, double& r, double& u, double& re, double& p)
+{
+    // I[w][v] of trace_project: its own reference wave, the u wave, the far wave
+    const double ref[4] = {rho_i, un_i, p_i, re_i}, mid[4] = {rho1, 0.0, p1, re1}, far[4] = {0.0, uo, po, 0.0};
+    double I[3][4];
+    for (int v = 0; v < 4; ++v) {
+        I[1][v] = mid[v];
+        I[0][v] = plus ? ref[v] : far[v];
+        I[2][v] = plus ? far[v] : ref[v];
+    }
+    trace_project(I, gam, un, cc, plus, r, u, re, p);
+}
+
 // Characteristic projection of trace_ppm (ppm.F90:537-623 for the plus state,
 // :637-734 for the minus state).  I[w][v] are the wave integrals of rho, un, p,
 // rhoe (v = 0..3) for waves w = u-c, u, u+c; gam is the gamc integral of the
