@@ -876,12 +876,19 @@ CASTRO_HD double uflatten(const L& ld, int i, int j, int k)
     for (int idir = 0; idir < 3; ++idir) {
         const int ex = idir == 0, ey = idir == 1, ez = idir == 2;
         const int qun = QU + idir;
-        double pr = ld.q(i + ex, j + ey, k + ez, QPRES);
-        double pl = ld.q(i - ex, j - ey, k - ez, QPRES);
-        double dp2 = ld.q(i + 2 * ex, j + 2 * ey, k + 2 * ez, QPRES) - ld.q(i - 2 * ex, j - 2 * ey, k - 2 * ez, QPRES);
-        double du = ld.q(i + ex, j + ey, k + ez, qun) - ld.q(i - ex, j - ey, k - ez, qun);
+        // both shifted stencils are read before the shift is known: one round of
+        // loads where indexing by the shift made the second depend on the first
+        double p[7], u[5];
+#pragma unroll
+        for (int m = -3; m <= 3; ++m) p[m + 3] = ld.q(i + m * ex, j + m * ey, k + m * ez, QPRES);
+#pragma unroll
+        for (int m = -2; m <= 2; ++m) u[m + 2] = ld.q(i + m * ex, j + m * ey, k + m * ez, qun);
+        double pr = p[4];
+        double pl = p[2];
+        double dp2 = p[5] - p[1];
+        double du = u[3] - u[1];
         double dp = pr - pl;
-        int s = (dp > 0.0) ? -1 : 1;   // s = -ishft
+        const bool left = dp > 0.0;    // the stencil shifted by one zone to the left (ishft = 1), else to the right
         double denom = DMAX(small_pres, fabs(dp2));
         double denominv = rcp(denom);
         double zeta = fabs(dp) * denominv;
@@ -890,12 +897,10 @@ CASTRO_HD double uflatten(const L& ld, int i, int j, int k)
         double tmp = DMIN(pr, pl);
         double chi = (fabs(dp) > shktst * tmp) ? tst : 0.0;
 
-        pr = ld.q(i + (1 + s) * ex, j + (1 + s) * ey, k + (1 + s) * ez, QPRES);
-        pl = ld.q(i + (s - 1) * ex, j + (s - 1) * ey, k + (s - 1) * ez, QPRES);
-        dp2 = ld.q(i + (2 + s) * ex, j + (2 + s) * ey, k + (2 + s) * ez, QPRES)
-            - ld.q(i + (s - 2) * ex, j + (s - 2) * ey, k + (s - 2) * ez, QPRES);
-        du = ld.q(i + (1 + s) * ex, j + (1 + s) * ey, k + (1 + s) * ez, qun)
-           - ld.q(i + (s - 1) * ex, j + (s - 1) * ey, k + (s - 1) * ez, qun);
+        pr = left ? p[3] : p[5];
+        pl = left ? p[1] : p[3];
+        dp2 = left ? p[4] - p[0] : p[6] - p[2];
+        du = left ? u[2] - u[0] : u[4] - u[2];
         dp = pr - pl;
         denom = DMAX(small_pres, fabs(dp2));
         denominv = rcp(denom);

@@ -432,15 +432,28 @@ __device__ __forceinline__ void ghost_body(const SimDev& S, const Work& w)
     const Reg R = q_region(I);
     double* Q = S.Q + B.offQ;
     const int is = ridx(R, ii, jj, kk), id = ridx(R, i, j, k);
+    // every component is read before the first is written: one round of loads
+    // (copied one by one each waited for its own, the arrays being one another's
+    // aliases for all the compiler knows)
+    constexpr int NQ = QF<NS>::N, NU = Dims<NS>::NVAR;
+    const bool inner = i >= I.dom_lo[0] - 1 && i <= I.dom_hi[0] + 1 && j >= I.dom_lo[1] - 1 && j <= I.dom_hi[1] + 1 &&
+                       k >= I.dom_lo[2] - 1 && k <= I.dom_hi[2] + 1;
+    const Reg R1 = u_region(I);
+    double* Ub = S.Ub + B.offUb;
+    double q[NQ], u[NU];
 #pragma unroll
-    for (int c = 0; c < QF<NS>::N; ++c) (Q + id)[R.plane(c)] = (Q + is)[R.plane(c)];
-    if (i >= I.dom_lo[0] - 1 && i <= I.dom_hi[0] + 1 && j >= I.dom_lo[1] - 1 && j <= I.dom_hi[1] + 1 &&
-        k >= I.dom_lo[2] - 1 && k <= I.dom_hi[2] + 1) {
-        const Reg R1 = u_region(I);
-        double* Ub = S.Ub + B.offUb;
-        const int is1 = ridx(R1, ii, jj, kk), id1 = ridx(R1, i, j, k);
+    for (int c = 0; c < NQ; ++c) q[c] = (Q + is)[R.plane(c)];
+    if (inner) {
+        const double* us = Ub + ridx(R1, ii, jj, kk);
 #pragma unroll
-        for (int n = 0; n < Dims<NS>::NVAR; ++n) (Ub + id1)[R1.plane(n)] = (Ub + is1)[R1.plane(n)];
+        for (int n = 0; n < NU; ++n) u[n] = us[R1.plane(n)];
+    }
+#pragma unroll
+    for (int c = 0; c < NQ; ++c) (Q + id)[R.plane(c)] = q[c];
+    if (inner) {
+        double* ud = Ub + ridx(R1, i, j, k);
+#pragma unroll
+        for (int n = 0; n < NU; ++n) ud[R1.plane(n)] = u[n];
     }
 }
 
@@ -714,6 +727,20 @@ __global__ void LB_TRACE2 k_trace2(SimDev S, const Work* wl)
 {
     trace_item<NS, 2>(S, wl[blockIdx.x]);
 }
+
+// Both passes in one launch, pass 2's items after pass 1's: the box entry
+// points' form while the two together are no more than one wave of pass 1's
+// blocks (three per SM), where a pass 2 launched behind pass 1 only adds its
+// latency
+template <int NS>
+__global__ void LB_TRACE k_trace_both(SimDev S, const Work* wl, int n)
+{
+    if ((int)blockIdx.x < n) trace_item<NS, 1>(S, wl[blockIdx.x]);
+    else trace_item<NS, 2>(S, wl[blockIdx.x - n]);
+}
+
+// whether the box entry points trace a box of n items a pass in one launch
+inline bool trace_in_one_launch(long long n) { return !CASTRO_TRACE_SPLIT || 2 * n <= 3 * 148; }
 
 // compute_flux on the face (i,j,k) normal to D: left zone i-e_D, right zone i
 // returns (GDPRES, Godunov velocity normal to the face)
@@ -1681,11 +1708,13 @@ __global__ void __launch_bounds__(BLOCK) k_box_prim(SimDev S, const Work* wl, Fa
     }
 }
 
-// fill_hydro_source into the caller's source FAB (Castro_hydro_nd.F90:411-439)
+// fill_hydro_source into the caller's source FAB (Castro_hydro_nd.F90:411-439).
+// Every operand is read before the first component is written: the arrays may
+// alias for all the compiler knows, and written one by one each component's
+// loads waited behind the last one's store.
 template <int NS>
-__global__ void __launch_bounds__(BLOCK) k_box_source(SimDev S, const Work* wl, Fab SRC)
+__device__ __forceinline__ void box_source_body(const SimDev& S, const Work& w, const Fab& SRC)
 {
-    const Work& w = wl[blockIdx.x];
     int b, sub, i, j, k;
     Reg R;
     if (!work_point(w, S, R_VALID, -1, b, sub, R, i, j, k)) return;
@@ -1704,13 +1733,15 @@ __global__ void __launch_bounds__(BLOCK) k_box_source(SimDev S, const Work* wl, 
         f0[d] = ridx(RX[d], i, j, k);
         f1[d] = ridx(RX[d], i + (d == 0), j + (d == 1), k + (d == 2));
     }
+    double src[NVAR];
 #pragma unroll
     for (int n = 0; n < NVAR; ++n) {
-        if (n == UTEMP) { SRC(i, j, k, n) = SRC(i, j, k, n) + 0.0 * volinv; continue; }
+        src[n] = SRC(i, j, k, n);
+        if (n == UTEMP) { src[n] = src[n] + 0.0 * volinv; continue; }
         const int c = n < UTEMP ? n : n - 1;
-        double s = SRC(i, j, k, n) + ((X[0] + f0[0])[RX[0].plane(c)] * a0 - (X[0] + f1[0])[RX[0].plane(c)] * a0
-                                    + (X[1] + f0[1])[RX[1].plane(c)] * a1 - (X[1] + f1[1])[RX[1].plane(c)] * a1
-                                    + (X[2] + f0[2])[RX[2].plane(c)] * a2 - (X[2] + f1[2])[RX[2].plane(c)] * a2) * volinv;
+        double s = src[n] + ((X[0] + f0[0])[RX[0].plane(c)] * a0 - (X[0] + f1[0])[RX[0].plane(c)] * a0
+                             + (X[1] + f0[1])[RX[1].plane(c)] * a1 - (X[1] + f1[1])[RX[1].plane(c)] * a1
+                             + (X[2] + f0[2])[RX[2].plane(c)] * a2 - (X[2] + f1[2])[RX[2].plane(c)] * a2) * volinv;
         if (n == UEINT) {
             const int P = NVAR - 1, V = NVAR;
             double pdivu = 0.5 * ((X[0] + f1[0])[RX[0].plane(P)] + (X[0] + f0[0])[RX[0].plane(P)]) *
@@ -1721,29 +1752,44 @@ __global__ void __launch_bounds__(BLOCK) k_box_source(SimDev S, const Work* wl, 
                                ((X[2] + f1[2])[RX[2].plane(V)] - (X[2] + f0[2])[RX[2].plane(V)]) / I.dx[2];
             s = s - pdivu;
         }
-        SRC(i, j, k, n) = s;
+        src[n] = s;
     }
+#pragma unroll
+    for (int n = 0; n < NVAR; ++n) SRC(i, j, k, n) = src[n];
 }
 
 // store_flux (Castro_hydro_nd.F90:330-338): dt * F * A on the faces of ebx[d]
 template <int NS>
-__global__ void __launch_bounds__(BLOCK) k_box_store_flux(SimDev S, const Work* wl, Fab FO0, Fab FO1, Fab FO2, double dt)
+__device__ __forceinline__ void box_flux_body(const SimDev& S, const Work& w, const Fab& FO, double dt)
 {
-    const Work& w = wl[blockIdx.x];
     int b, d, i, j, k;
     Reg R;
-    if (!work_point(w, S, R_EBX, -1, b, d, R, i, j, k)) return;
+    if (!FO.p || !work_point(w, S, R_EBX, -1, b, d, R, i, j, k)) return;
     const BoxDev& B = S.boxes[b];
     const InstDev& I = S.inst[B.inst];
-    const Fab& FO = d == 0 ? FO0 : d == 1 ? FO1 : FO2;
-    if (!FO.p) return;
     const double area = d == 0 ? I.dx[1] * I.dx[2] : d == 1 ? I.dx[0] * I.dx[2] : I.dx[0] * I.dx[1];
-    const double* X = S.Fx + B.offFx[d];
-    const int f = ridx(R, i, j, k);
+    const double* X = S.Fx + B.offFx[d] + ridx(R, i, j, k);
+    constexpr int NVAR = Dims<NS>::NVAR;
+    double F[NVAR];
 #pragma unroll
-    for (int n = 0; n < Dims<NS>::NVAR; ++n) {
-        double F = (n == UTEMP) ? 0.0 : (X + f)[R.plane(n < UTEMP ? n : n - 1)];
-        FO(i, j, k, n) = dt * F * area;
+    for (int n = 0; n < NVAR; ++n) F[n] = (n == UTEMP) ? 0.0 : X[R.plane(n < UTEMP ? n : n - 1)];
+#pragma unroll
+    for (int n = 0; n < NVAR; ++n) FO(i, j, k, n) = dt * F[n] * area;
+}
+
+// the box entry points' outputs in one launch: the source's items, then (nf of
+// them, when the caller wants fluxes) store_flux's
+template <int NS>
+__global__ void __launch_bounds__(BLOCK) k_box_out(SimDev S, const Work* wv, int nv, const Work* wf, Fab SRC, Fab FO0, Fab FO1,
+                                                   Fab FO2, double dt)
+{
+    if ((int)blockIdx.x < nv) {
+        box_source_body<NS>(S, wv[blockIdx.x], SRC);
+    } else {
+        const Work& w = wf[blockIdx.x - nv];
+        if (w.sub == 0) box_flux_body<NS>(S, w, FO0, dt);
+        else if (w.sub == 1) box_flux_body<NS>(S, w, FO1, dt);
+        else box_flux_body<NS>(S, w, FO2, dt);
     }
 }
 
@@ -2449,9 +2495,12 @@ int step_impl(castro_sim* s)
         plain_step<NS>(s);
         // per box: estdt, fill_sborder, Saxpy and 4 x 4 clean kernels, plus construct_hydro_source's
         // 36 per-routine launches or the fused box path's kernels (prim, prep, trace (x2), riemann1-3, source)
-        const int per_box = 19 + (s->mode == CASTRO_MODE_PLAIN ? 36 : 6 + (CASTRO_TRACE_SPLIT ? 2 : 1));
         s->launches = 0;
-        for (int in = 0; in < s->ninst; ++in) s->launches += per_box * (int)s->inst_boxes[in].size();
+        for (const BoxDev& B : s->hboxes) {
+            long long nt = 0;
+            for (int d = 0; d < 3; ++d) nt += (npts_reg(B.lo, B.hi, R_SEG, d) + BLOCK - 1) / BLOCK;
+            s->launches += 19 + (s->mode == CASTRO_MODE_PLAIN ? 36 : 6 + (trace_in_one_launch(nt) ? 1 : 2));
+        }
         return castro_last_error();
     }
     if (!s->dt_ready) {
@@ -3334,20 +3383,24 @@ int box_hydro_launch(const BoxPlan& P, double* base, long long meta_doubles, con
     const Work* W = work;
     CASTRO_EOS_LAUNCH(k_box_prim, NS, nblocks[NL_G4], BLOCK, 0, cs, S, W + NLs.first[NL_G4], make_fab(sb, sb_lo, sb_hi));
     k_prep<NS><<<nblocks[NL_G1], BLOCK, 0, cs>>>(S, W + NLs.first[NL_G1]);
-    k_trace<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
-    if (CASTRO_TRACE_SPLIT) k_trace2<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+    if (!CASTRO_TRACE_SPLIT) {
+        k_trace<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+    } else if (trace_in_one_launch(nblocks[NL_TRACE])) {
+        k_trace_both<NS><<<2 * nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE], nblocks[NL_TRACE]);
+    } else {
+        k_trace<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+        k_trace2<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+    }
     k_riemann1<NS><<<nblocks[NL_TBX], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TBX]);
     k_riemann2<NS><<<nblocks[NL_TBX], BLOCK, R2Slot<NS>::BYTES, cs>>>(S, W + NLs.first[NL_TBX]);
     k_riemann3<NS><<<nblocks[NL_EBX], BLOCK, R3Slot<NS>::BYTES, cs>>>(S, W + NLs.first[NL_EBX]);
-    k_box_source<NS><<<nblocks[NL_VALID], BLOCK, 0, cs>>>(S, W + NLs.first[NL_VALID], make_fab(source, sr_lo, sr_hi));
-    if (fo) {
-        Fab F[3];
-        for (int d = 0; d < 3; ++d) {
-            F[d] = fo[d] ? make_fab(fo[d], fo_lo + 3 * d, fo_hi + 3 * d) : Fab{};
-            if (!fo[d]) F[d].p = nullptr;
-        }
-        k_box_store_flux<NS><<<nblocks[NL_EBX], BLOCK, 0, cs>>>(S, W + NLs.first[NL_EBX], F[0], F[1], F[2], dt);
-    }
+    Fab F[3] = {};
+    if (fo)
+        for (int d = 0; d < 3; ++d)
+            if (fo[d]) F[d] = make_fab(fo[d], fo_lo + 3 * d, fo_hi + 3 * d);
+    k_box_out<NS><<<nblocks[NL_VALID] + (fo ? nblocks[NL_EBX] : 0), BLOCK, 0, cs>>>(
+        S, W + NLs.first[NL_VALID], nblocks[NL_VALID], W + NLs.first[NL_EBX], make_fab(source, sr_lo, sr_hi), F[0], F[1], F[2],
+        dt);
     check_launch(who);
     return castro_last_error();
 }
