@@ -352,6 +352,20 @@ __device__ __forceinline__ double block_min(double m)
 // fused kernels
 // ---------------------------------------------------------------------------
 
+// Programmatic dependent launch, taken by the box entry points (launch_behind):
+// a stage's blocks may be placed on the SMs once every block of the stage
+// before has begun, so that the launch and the ramp of one stage lie under the
+// tail of the other; they touch nothing before that stage has completed
+// (griddepcontrol.wait waits for the whole grid and its writes).  A kernel
+// launched without the attribute runs straight through: the batched step keeps
+// its graph's ordinary edges, which measured faster there (16^3 66.7 us against
+// 70.2 with programmatic edges, 13 species 64^3 789 against 815, others equal).
+__device__ __forceinline__ void stage_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // front: clean_state(S_old) -> S_new base; clean_state(Sborder); ctoprim
 template <int NS, bool COUL>
 __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
@@ -398,6 +412,7 @@ __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
 template <int NS, bool COUL>
 __global__ void LB_EOS k_front(SimDev S, const Work* wl)
 {
+    stage_begin();
     front_body<NS, COUL>(S, wl[blockIdx.x]);
 }
 
@@ -460,6 +475,7 @@ __device__ __forceinline__ void ghost_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void __launch_bounds__(BLOCK) k_ghost(SimDev S, const Work* wl)
 {
+    stage_begin();
     ghost_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -499,6 +515,7 @@ __device__ __forceinline__ void prep_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void __launch_bounds__(BLOCK) k_prep(SimDev S, const Work* wl)
 {
+    stage_begin();
     prep_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -719,12 +736,14 @@ __device__ __forceinline__ void trace_item(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void LB_TRACE k_trace(SimDev S, const Work* wl)
 {
+    stage_begin();
     trace_item<NS, CASTRO_TRACE_SPLIT ? 1 : 3>(S, wl[blockIdx.x]);
 }
 
 template <int NS>
 __global__ void LB_TRACE2 k_trace2(SimDev S, const Work* wl)
 {
+    stage_begin();
     trace_item<NS, 2>(S, wl[blockIdx.x]);
 }
 
@@ -735,6 +754,7 @@ __global__ void LB_TRACE2 k_trace2(SimDev S, const Work* wl)
 template <int NS>
 __global__ void LB_TRACE k_trace_both(SimDev S, const Work* wl, int n)
 {
+    stage_begin();
     if ((int)blockIdx.x < n) trace_item<NS, 1>(S, wl[blockIdx.x]);
     else trace_item<NS, 2>(S, wl[blockIdx.x - n]);
 }
@@ -805,6 +825,7 @@ __device__ __forceinline__ void riemann1_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void LB_RIEMANN k_riemann1(SimDev S, const Work* wl)
 {
+    stage_begin();
     riemann1_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -951,6 +972,7 @@ __device__ __forceinline__ void riemann2_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void LB_RIEMANN k_riemann2(SimDev S, const Work* wl)
 {
+    stage_begin();
     riemann2_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -1146,6 +1168,7 @@ __device__ __forceinline__ void riemann3_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void LB_R3 k_riemann3(SimDev S, const Work* wl)
 {
+    stage_begin();
     riemann3_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -1442,6 +1465,7 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
 template <int NS, bool COUL>
 __global__ void LB_EOS k_update(SimDev S, const Work* wl)
 {
+    stage_begin();
     update_body<NS, COUL>(S, wl[blockIdx.x]);
 }
 
@@ -1504,6 +1528,7 @@ __device__ __forceinline__ void next_dt(InstState& st, int first)
 
 __global__ void k_dt(SimDev S, int ninst, int first)
 {
+    stage_begin();
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ninst) return;
     next_dt(S.st[n], first);
@@ -1674,6 +1699,7 @@ __global__ void __launch_bounds__(BLOCK) k_fill_sborder(SimDev S, int b, double*
 template <int NS, bool COUL>
 __global__ void __launch_bounds__(BLOCK) k_box_prim(SimDev S, const Work* wl, Fab SB)
 {
+    stage_begin();
     const Work& w = wl[blockIdx.x];
     int b, sub, i, j, k;
     Reg R;
@@ -1783,6 +1809,7 @@ template <int NS>
 __global__ void __launch_bounds__(BLOCK) k_box_out(SimDev S, const Work* wv, int nv, const Work* wf, Fab SRC, Fab FO0, Fab FO1,
                                                    Fab FO2, double dt)
 {
+    stage_begin();
     if ((int)blockIdx.x < nv) {
         box_source_body<NS>(S, wv[blockIdx.x], SRC);
     } else {
@@ -2025,12 +2052,37 @@ void build_ghost_work(castro_sim* s)
         cuda_ok(cudaMemcpy(s->w_ghost, w.data(), w.size() * sizeof(Work), cudaMemcpyHostToDevice), "ghost work list copy");
 }
 
+// Launch of a stage behind the kernel before it in the stream, its blocks placed
+// early (stage_begin).  Eight launches of a few microseconds each make a box
+// call: box of 32^3, 2 species, B200: 99.4 -> 89.1 us, 16^3 with 13 species
+// 99.7 -> 91.6.
+template <class... P, class... A>
+void launch_behind(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Launch of a kernel that calls the EOS: the instantiation with or without the
 // Coulomb corrections, as the library is set (castro_set_coulomb_corrections).
 #define CASTRO_EOS_LAUNCH(K, NS, GRID, BLK, SMEM, ST, ...)                         \
     do {                                                                           \
         if (coulomb_on()) K<NS, true><<<GRID, BLK, SMEM, ST>>>(__VA_ARGS__);        \
         else K<NS, false><<<GRID, BLK, SMEM, ST>>>(__VA_ARGS__);                     \
+    } while (0)
+#define CASTRO_EOS_LAUNCH_BEHIND(K, NS, GRID, BLK, SMEM, ST, ...)                   \
+    do {                                                                           \
+        if (coulomb_on()) launch_behind(K<NS, true>, GRID, BLK, SMEM, ST, __VA_ARGS__);   \
+        else launch_behind(K<NS, false>, GRID, BLK, SMEM, ST, __VA_ARGS__);               \
     } while (0)
 
 // riemann23's column tiles over every instance domain; its shared memory
@@ -3266,6 +3318,7 @@ struct NoallocLists {
 __global__ void k_noalloc_setup(BoxDev B, InstDev I, InstState st, NoallocLists NLs, BoxDev* dB, InstDev* dI,
                                 InstState* dS, Work* work)
 {
+    stage_begin();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) {
         *dB = B;
@@ -3381,26 +3434,26 @@ int box_hydro_launch(const BoxPlan& P, double* base, long long meta_doubles, con
     S.boxes = dB; S.dom = dB; S.inst = dI; S.st = dS;   // the box is the instance domain
     S.Ub = pools; S.Q = pools; S.Div = pools; S.Tr = pools; S.F1 = pools; S.F2 = pools; S.Fx = pools;
     const Work* W = work;
-    CASTRO_EOS_LAUNCH(k_box_prim, NS, nblocks[NL_G4], BLOCK, 0, cs, S, W + NLs.first[NL_G4], make_fab(sb, sb_lo, sb_hi));
-    k_prep<NS><<<nblocks[NL_G1], BLOCK, 0, cs>>>(S, W + NLs.first[NL_G1]);
+    CASTRO_EOS_LAUNCH_BEHIND(k_box_prim, NS, nblocks[NL_G4], BLOCK, 0, cs, S, W + NLs.first[NL_G4],
+                             make_fab(sb, sb_lo, sb_hi));
+    launch_behind(k_prep<NS>, nblocks[NL_G1], BLOCK, 0, cs, S, W + NLs.first[NL_G1]);
     if (!CASTRO_TRACE_SPLIT) {
-        k_trace<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+        launch_behind(k_trace<NS>, nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE]);
     } else if (trace_in_one_launch(nblocks[NL_TRACE])) {
-        k_trace_both<NS><<<2 * nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE], nblocks[NL_TRACE]);
+        launch_behind(k_trace_both<NS>, 2 * nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE], nblocks[NL_TRACE]);
     } else {
-        k_trace<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
-        k_trace2<NS><<<nblocks[NL_TRACE], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TRACE]);
+        launch_behind(k_trace<NS>, nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE]);
+        launch_behind(k_trace2<NS>, nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE]);
     }
-    k_riemann1<NS><<<nblocks[NL_TBX], BLOCK, 0, cs>>>(S, W + NLs.first[NL_TBX]);
-    k_riemann2<NS><<<nblocks[NL_TBX], BLOCK, R2Slot<NS>::BYTES, cs>>>(S, W + NLs.first[NL_TBX]);
-    k_riemann3<NS><<<nblocks[NL_EBX], BLOCK, R3Slot<NS>::BYTES, cs>>>(S, W + NLs.first[NL_EBX]);
+    launch_behind(k_riemann1<NS>, nblocks[NL_TBX], BLOCK, 0, cs, S, W + NLs.first[NL_TBX]);
+    launch_behind(k_riemann2<NS>, nblocks[NL_TBX], BLOCK, R2Slot<NS>::BYTES, cs, S, W + NLs.first[NL_TBX]);
+    launch_behind(k_riemann3<NS>, nblocks[NL_EBX], BLOCK, R3Slot<NS>::BYTES, cs, S, W + NLs.first[NL_EBX]);
     Fab F[3] = {};
     if (fo)
         for (int d = 0; d < 3; ++d)
             if (fo[d]) F[d] = make_fab(fo[d], fo_lo + 3 * d, fo_hi + 3 * d);
-    k_box_out<NS><<<nblocks[NL_VALID] + (fo ? nblocks[NL_EBX] : 0), BLOCK, 0, cs>>>(
-        S, W + NLs.first[NL_VALID], nblocks[NL_VALID], W + NLs.first[NL_EBX], make_fab(source, sr_lo, sr_hi), F[0], F[1], F[2],
-        dt);
+    launch_behind(k_box_out<NS>, nblocks[NL_VALID] + (fo ? nblocks[NL_EBX] : 0), BLOCK, 0, cs, S, W + NLs.first[NL_VALID],
+                  nblocks[NL_VALID], W + NLs.first[NL_EBX], make_fab(source, sr_lo, sr_hi), F[0], F[1], F[2], dt);
     check_launch(who);
     return castro_last_error();
 }
