@@ -278,11 +278,22 @@ void apply_av_impl(const int* lo, const int* hi, int idir, double dxd, Fab DIV, 
         else if (idir == 1) ds = DIV(i, j, k, 0) + DIV(i + 1, j, k, 0) + DIV(i, j, k + 1, 0) + DIV(i + 1, j, k, 0);
         else ds = DIV(i, j, k, 0) + DIV(i + 1, j, k, 0) + DIV(i, j + 1, k, 0) + DIV(i + 1, j + 1, k, 0);
         const int ex = idir == 0, ey = idir == 1, ez = idir == 2;
+        // (here and below: every component is read before the first is written;
+        // the FABs may alias for all the compiler knows, and each component's
+        // loads would wait behind the last one's store)
+        constexpr int NVAR = Dims<NS>::NVAR;
+        double du[NVAR], f[NVAR];
 #pragma unroll
-        for (int n = 0; n < Dims<NS>::NVAR; ++n) {
+        for (int n = 0; n < NVAR; ++n) {
             if (n == UTEMP) continue;
-            double div1 = av_term(ds, U(i, j, k, n) - U(i - ex, j - ey, k - ez, n));
-            FX(i, j, k, n) = FX(i, j, k, n) + dxd * div1;
+            du[n] = U(i, j, k, n) - U(i - ex, j - ey, k - ez, n);
+            f[n] = FX(i, j, k, n);
+        }
+#pragma unroll
+        for (int n = 0; n < NVAR; ++n) {
+            if (n == UTEMP) continue;
+            double div1 = av_term(ds, du[n]);
+            FX(i, j, k, n) = f[n] + dxd * div1;
         }
     });
 }
@@ -291,12 +302,15 @@ template <int NS>
 void normalize_species_fluxes_impl(const int* lo, const int* hi, Fab FX)
 {
     launch_box("normalize_species_fluxes", lo, hi, [=] __device__(int i, int j, int k) {
-        double sum = 0.0;
+        double f[NS], sum = 0.0;
 #pragma unroll
-        for (int n = 0; n < NS; ++n) sum = sum + FX(i, j, k, UFS + n);
+        for (int n = 0; n < NS; ++n) {
+            f[n] = FX(i, j, k, UFS + n);
+            sum = sum + f[n];
+        }
         double fac = (sum != 0.0) ? FX(i, j, k, URHO) / sum : 1.0;
 #pragma unroll
-        for (int n = 0; n < NS; ++n) FX(i, j, k, UFS + n) = FX(i, j, k, UFS + n) * fac;
+        for (int n = 0; n < NS; ++n) FX(i, j, k, UFS + n) = f[n] * fac;
     });
 }
 
@@ -304,8 +318,13 @@ template <int NS>
 void store_flux_impl(const int* lo, const int* hi, Fab FO, Fab FI, Fab A, double dt)
 {
     launch_box("store_flux", lo, hi, [=] __device__(int i, int j, int k) {
+        constexpr int NVAR = Dims<NS>::NVAR;
+        const double a = A(i, j, k, 0);
+        double f[NVAR];
 #pragma unroll
-        for (int n = 0; n < Dims<NS>::NVAR; ++n) FO(i, j, k, n) = dt * FI(i, j, k, n) * A(i, j, k, 0);
+        for (int n = 0; n < NVAR; ++n) f[n] = FI(i, j, k, n);
+#pragma unroll
+        for (int n = 0; n < NVAR; ++n) FO(i, j, k, n) = dt * f[n] * a;
     });
 }
 
@@ -314,12 +333,17 @@ void fill_hydro_source_impl(const int* lo, const int* hi, Fab SRC, Fab F0, Fab F
                             Fab A0, Fab A1, Fab A2, Fab V, double dx0, double dx1, double dx2)
 {
     launch_box("fill_hydro_source", lo, hi, [=] __device__(int i, int j, int k) {
-        for (int n = 0; n < Dims<NS>::NVAR; ++n) {
-            double volinv = 1.0 / V(i, j, k, 0);
-            SRC(i, j, k, n) = SRC(i, j, k, n) +
-                (F0(i, j, k, n) * A0(i, j, k, 0) - F0(i + 1, j, k, n) * A0(i + 1, j, k, 0)
-               + F1(i, j, k, n) * A1(i, j, k, 0) - F1(i, j + 1, k, n) * A1(i, j + 1, k, 0)
-               + F2(i, j, k, n) * A2(i, j, k, 0) - F2(i, j, k + 1, n) * A2(i, j, k + 1, 0)) * volinv;
+        constexpr int NVAR = Dims<NS>::NVAR;
+        const double volinv = 1.0 / V(i, j, k, 0);
+        const double a0l = A0(i, j, k, 0), a0h = A0(i + 1, j, k, 0), a1l = A1(i, j, k, 0), a1h = A1(i, j + 1, k, 0),
+                     a2l = A2(i, j, k, 0), a2h = A2(i, j, k + 1, 0);
+        double src[NVAR];
+#pragma unroll
+        for (int n = 0; n < NVAR; ++n) {
+            src[n] = SRC(i, j, k, n) +
+                (F0(i, j, k, n) * a0l - F0(i + 1, j, k, n) * a0h
+               + F1(i, j, k, n) * a1l - F1(i, j + 1, k, n) * a1h
+               + F2(i, j, k, n) * a2l - F2(i, j, k + 1, n) * a2h) * volinv;
             if (n == UEINT) {
                 double pdivu = 0.5 * (Q0(i + 1, j, k, GDPRES) + Q0(i, j, k, GDPRES)) *
                                    (Q0(i + 1, j, k, GDU) - Q0(i, j, k, GDU)) / dx0 +
@@ -327,9 +351,11 @@ void fill_hydro_source_impl(const int* lo, const int* hi, Fab SRC, Fab F0, Fab F
                                    (Q1(i, j + 1, k, GDV) - Q1(i, j, k, GDV)) / dx1 +
                                0.5 * (Q2(i, j, k + 1, GDPRES) + Q2(i, j, k, GDPRES)) *
                                    (Q2(i, j, k + 1, GDW) - Q2(i, j, k, GDW)) / dx2;
-                SRC(i, j, k, n) = SRC(i, j, k, n) - pdivu;
+                src[n] = src[n] - pdivu;
             }
         }
+#pragma unroll
+        for (int n = 0; n < NVAR; ++n) SRC(i, j, k, n) = src[n];
     });
 }
 

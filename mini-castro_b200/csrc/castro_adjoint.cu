@@ -107,14 +107,19 @@ __device__ __forceinline__ void ld_state(const Fab& f, int i, int j, int k, doub
 template <int NS>
 __device__ __forceinline__ void add_state(const Fab& f, int i, int j, int k, const double* s)
 {
-    f(i, j, k, QRHO) += s[SRHO];
-    f(i, j, k, QU) += s[SU];
-    f(i, j, k, QV) += s[SV];
-    f(i, j, k, QW) += s[SW];
-    f(i, j, k, QPRES) += s[SPRES];
-    f(i, j, k, QREINT) += s[SREI];
+    // every component is read before the first is written (here and in the other
+    // accumulations below): the FABs may alias for all the compiler knows, and
+    // added one by one each load waited behind the last component's store
+    double t[Dims<NS>::NQS];
+    ld_state<NS>(f, i, j, k, t);
+    f(i, j, k, QRHO) = t[SRHO] + s[SRHO];
+    f(i, j, k, QU) = t[SU] + s[SU];
+    f(i, j, k, QV) = t[SV] + s[SV];
+    f(i, j, k, QW) = t[SW] + s[SW];
+    f(i, j, k, QPRES) = t[SPRES] + s[SPRES];
+    f(i, j, k, QREINT) = t[SREI] + s[SREI];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) f(i, j, k, QFS + n) += s[SX + n];
+    for (int n = 0; n < NS; ++n) f(i, j, k, QFS + n) = t[SX + n] + s[SX + n];
 }
 
 template <int NS>
@@ -594,13 +599,19 @@ void apply_av_adj_impl(const int* lo, const int* hi, int idir, double dxd, Fab D
         const int ex = idir == 0, ey = idir == 1, ez = idir == 2;
         const double d1 = 0.25 * ds;
         const double div1 = 0.1 * DMIN(0.0, d1);
-        double div1b = 0.0;
+        double div1b = 0.0, fxb[Dims<NS>::NVAR], dU[Dims<NS>::NVAR];
 #pragma unroll
         for (int n = 0; n < Dims<NS>::NVAR; ++n) {
             if (n == UTEMP) continue;
-            const double g = FXB(i, j, k, n) * dxd;
+            fxb[n] = FXB(i, j, k, n);
+            dU[n] = U(i, j, k, n) - U(i - ex, j - ey, k - ez, n);
+        }
+#pragma unroll
+        for (int n = 0; n < Dims<NS>::NVAR; ++n) {
+            if (n == UTEMP) continue;
+            const double g = fxb[n] * dxd;
             if (g == 0.0) continue;
-            const double du = U(i, j, k, n) - U(i - ex, j - ey, k - ez, n);
+            const double du = dU[n];
             aadd(&UB(i, j, k, n), g * div1);
             aadd(&UB(i - ex, j - ey, k - ez, n), -g * div1);
             div1b += g * du;
@@ -629,13 +640,17 @@ void normalize_species_fluxes_adj_impl(const int* lo, const int* hi, Fab FX, Fab
         if (sum == 0.0) return;
         const double fr = FX(i, j, k, URHO);
         const double fac = fr / sum;
-        double facb = 0.0;
+        double facb = 0.0, fxb[NS];
+        const double frb = FXB(i, j, k, URHO);
 #pragma unroll
-        for (int n = 0; n < NS; ++n) facb += FXB(i, j, k, UFS + n) * FX(i, j, k, UFS + n);
+        for (int n = 0; n < NS; ++n) {
+            fxb[n] = FXB(i, j, k, UFS + n);
+            facb += fxb[n] * FX(i, j, k, UFS + n);
+        }
         const double sumb = -(facb / sum) * fac;
-        FXB(i, j, k, URHO) += facb / sum;
+        FXB(i, j, k, URHO) = frb + facb / sum;
 #pragma unroll
-        for (int n = 0; n < NS; ++n) FXB(i, j, k, UFS + n) = FXB(i, j, k, UFS + n) * fac + sumb;
+        for (int n = 0; n < NS; ++n) FXB(i, j, k, UFS + n) = fxb[n] * fac + sumb;
     });
 }
 
@@ -646,16 +661,22 @@ void fill_hydro_source_adj_impl(const int* lo, const int* hi, Fab SRCB, Fab Q0, 
 {
     launch_box("fill_hydro_source_adj", lo, hi, [=] __device__(int i, int j, int k) {
         const double volinv = 1.0 / V(i, j, k, 0);
+        const double a0l = A0(i, j, k, 0), a0h = A0(i + 1, j, k, 0), a1l = A1(i, j, k, 0), a1h = A1(i, j + 1, k, 0),
+                     a2l = A2(i, j, k, 0), a2h = A2(i, j, k + 1, 0);
+        double srcb[Dims<NS>::NVAR];
+#pragma unroll
+        for (int n = 0; n < Dims<NS>::NVAR; ++n) srcb[n] = SRCB(i, j, k, n);
+#pragma unroll
         for (int n = 0; n < Dims<NS>::NVAR; ++n) {
-            const double sb = SRCB(i, j, k, n);
+            const double sb = srcb[n];
             if (sb == 0.0) continue;
             const double t = sb * volinv;
-            aadd(&F0B(i, j, k, n), t * A0(i, j, k, 0));
-            aadd(&F0B(i + 1, j, k, n), -t * A0(i + 1, j, k, 0));
-            aadd(&F1B(i, j, k, n), t * A1(i, j, k, 0));
-            aadd(&F1B(i, j + 1, k, n), -t * A1(i, j + 1, k, 0));
-            aadd(&F2B(i, j, k, n), t * A2(i, j, k, 0));
-            aadd(&F2B(i, j, k + 1, n), -t * A2(i, j, k + 1, 0));
+            aadd(&F0B(i, j, k, n), t * a0l);
+            aadd(&F0B(i + 1, j, k, n), -t * a0h);
+            aadd(&F1B(i, j, k, n), t * a1l);
+            aadd(&F1B(i, j + 1, k, n), -t * a1h);
+            aadd(&F2B(i, j, k, n), t * a2l);
+            aadd(&F2B(i, j, k + 1, n), -t * a2h);
             if (n == UEINT) {
                 const double pb = -sb;   // source -= pdivu
                 {
@@ -1180,13 +1201,18 @@ void begin_step(castro_adj* a, const Arr& Vin)
     clean(a->dom, a->P->A);
 }
 
-__global__ void k_saxpy_box(BoxRange r, Fab A, Fab S, Fab B, int nv, double dt)
+template <int NV>
+__global__ void k_saxpy_box(BoxRange r, Fab A, Fab S, Fab B, double dt)
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
     int i, j, k;
     range_point(r, t, i, j, k);
-    for (int n = 0; n < nv; ++n) B(i, j, k, n) = A(i, j, k, n) + dt * S(i, j, k, n);
+    double a[NV], s[NV];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) { a[n] = A(i, j, k, n); s[n] = S(i, j, k, n); }
+#pragma unroll
+    for (int n = 0; n < NV; ++n) B(i, j, k, n) = a[n] + dt * s[n];
 }
 
 // the forward of one step on the working box from the domain's cleaned S_old
@@ -1252,27 +1278,34 @@ void forward_step(castro_adj* a, double dt)
                       a->area[2].p, a->gebx[2].lo, a->gebx[2].hi, a->vol.p, bx.lo, bx.hi, a->dx, dt);
     {
         BoxRange r = make_range(bx.lo, bx.hi);                      // B = A + dt * src on the working box
-        k_saxpy_box<<<(unsigned)((r.n + 255) / 256), 256, 0, st>>>(r, a->P->A.fab(), a->P->src.fab(), a->P->Bs.fab(),
-                                                                     Dims<NS>::NVAR, dt);
+        k_saxpy_box<Dims<NS>::NVAR><<<(unsigned)((r.n + 255) / 256), 256, 0, st>>>(r, a->P->A.fab(), a->P->src.fab(),
+                                                                                   a->P->Bs.fab(), dt);
     }
     copy(a->P->Cs, a->P->Bs, st);
     clean(bx, a->P->Cs);                                          // clean_state(S_new), Castro_advance.cpp
 }
 
-__global__ void k_copy_box(BoxRange r, Fab D, Fab S, int nv)
+template <int NV>
+__global__ void k_copy_box(BoxRange r, Fab D, Fab S)
 {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= r.n) return;
     int i, j, k;
     range_point(r, t, i, j, k);
-    for (int n = 0; n < nv; ++n) D(i, j, k, n) = S(i, j, k, n);
+    double s[NV];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) s[n] = S(i, j, k, n);
+#pragma unroll
+    for (int n = 0; n < NV; ++n) D(i, j, k, n) = s[n];
 }
 
 // V_{n+1} = clean(C) on the working box of the domain-sized Vout
 void finish_step(castro_adj* a, const Arr& Vout)
 {
     BoxRange r = make_range(a->bx.lo, a->bx.hi);
-    k_copy_box<<<(unsigned)((r.n + 255) / 256), 256, 0, a->st>>>(r, Vout.fab(), a->P->Cs.fab(), a->nv);
+    const unsigned nb = (unsigned)((r.n + 255) / 256);
+    if (a->ns == 2) k_copy_box<Dims<2>::NVAR><<<nb, 256, 0, a->st>>>(r, Vout.fab(), a->P->Cs.fab());
+    else k_copy_box<Dims<13>::NVAR><<<nb, 256, 0, a->st>>>(r, Vout.fab(), a->P->Cs.fab());
     clean(a->bx, Vout);                                        // post_timestep clean_state, Castro.cpp:369
 }
 
@@ -1550,13 +1583,18 @@ void reverse_step(castro_adj* a, double dt)
     {
         Fab BB = a->Vb.fab(), AB = a->Ab.fab(), SB = a->srcb.fab(), S = a->P->src.fab();
         launch_sum("adj saxpy", bx.lo, bx.hi, [=] __device__(int i, int j, int k) -> double {
-            double s = 0.0;
+            constexpr int NV = Dims<NS>::NVAR;
+            double s = 0.0, b[NV], ab[NV];
 #pragma unroll
-            for (int n = 0; n < Dims<NS>::NVAR; ++n) {
-                double b = BB(i, j, k, n);
-                AB(i, j, k, n) += b;
-                SB(i, j, k, n) = dt * b;
-                s += S(i, j, k, n) * b;
+            for (int n = 0; n < NV; ++n) {
+                b[n] = BB(i, j, k, n);
+                ab[n] = AB(i, j, k, n);
+                s += S(i, j, k, n) * b[n];
+            }
+#pragma unroll
+            for (int n = 0; n < NV; ++n) {
+                AB(i, j, k, n) = ab[n] + b[n];
+                SB(i, j, k, n) = dt * b[n];
             }
             return s;
         }, sc + 9);
