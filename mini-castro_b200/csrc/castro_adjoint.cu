@@ -163,6 +163,8 @@ constexpr int PART_MAX = 1 << 20;
 constexpr int MAX_DEVICES = 64;
 double* g_part_dev[MAX_DEVICES] = {};
 double* g_part = nullptr;   // the current device's buffer (set by part_buffer)
+// the partial sums of the lane whose work is being launched (Lanes), when one is
+double* g_part_lane = nullptr;
 
 __global__ void k_finish_sum(const double* part, int nb, double* out0, double* out1)
 {
@@ -179,13 +181,17 @@ __global__ void k_finish_sum(const double* part, int nb, double* out0, double* o
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += red[0][w]; b += red[1][w]; }
-        if (out0) *out0 += a;
-        if (out1) *out1 += b;
+        if (out0) atomicAdd(out0, a);   // lanes share scalars
+        if (out1) atomicAdd(out1, b);
     }
 }
 
 bool part_buffer()
 {
+    if (g_part_lane) {
+        g_part = g_part_lane;
+        return true;
+    }
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
         set_error(CASTRO_ERR_CUDA, "adjoint: current device");
@@ -421,8 +427,7 @@ void trace_adj_dir(const int* lo, const int* hi, int vl, int vh, Fab Q, Fab QA, 
         double dtdxb_l = 0.0;
         double fb = trace_zone_adj<NS, D>(ld, sk, i, j, k, dtdx, flatn, hp ? qpb : nullptr, hm ? qmb : nullptr, dtdxb_l);
         if (FLB.p) {
-            if (D == 0) FLB(i, j, k, 0) = fb;
-            else FLB(i, j, k, 0) += fb;
+            FLB(i, j, k, 0) = fb;
         } else {
             uflatten_adj(ld, sk, i, j, k, fb);
         }
@@ -433,12 +438,12 @@ void trace_adj_dir(const int* lo, const int* hi, int vl, int vh, Fab Q, Fab QA, 
 // the flattening reverse of every zone with the adjoint summed over the three
 // trace directions (uflatten_adj is linear in that adjoint)
 template <int NS>
-void uflatten_adj_zones(const int* lo, const int* hi, Fab Q, Fab QA, Fab QB, Fab QAB, Fab FLB)
+void uflatten_adj_zones(const int* lo, const int* hi, Fab Q, Fab QA, Fab QB, Fab QAB, Fab FL0, Fab FL1, Fab FL2)
 {
     launch_box("uflatten_adj zones", lo, hi, [=] __device__(int i, int j, int k) {
         QLoad ld{Q, QA};
         AtomicSink sk{QB, QAB};
-        uflatten_adj(ld, sk, i, j, k, FLB(i, j, k, 0));
+        uflatten_adj(ld, sk, i, j, k, FL0(i, j, k, 0) + FL1(i, j, k, 0) + FL2(i, j, k, 0));
     });
 }
 
@@ -934,7 +939,12 @@ struct castro_adj {
     Prim* P = nullptr;
     Arr V, area[3], vol, Vfinal;
     // adjoint
-    Arr flb;   // adjoint of the flattening coefficient, summed over the trace directions
+    Arr flb;   // adjoint of the flattening coefficient from the x trace (y, z: component 0 of qrb[1], qrb[2])
+    // Lanes: independent launches of one stage (its three directions) run on
+    // three streams, lane 0 being st
+    cudaStream_t lane[2] = {nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
+    double* part[3] = {nullptr, nullptr, nullptr};   // partial sums of each lane
     Arr Vb, Ab, Sbb, qb, qab, divb, qmb[3][3], qpb[3][3], F1b[3], G1b[3], F2b[3][3], G2b[3][3], qlb[3], qrb[3];
     Arr fluxb[3], qeb[3], srcb;
     // per-zone flux-record adjoints of the zone-based transverse reverses:
@@ -959,6 +969,41 @@ struct StreamScope {
     cudaStream_t saved;
     explicit StreamScope(cudaStream_t s) : saved(stream()) { castro_set_stream(s); }
     ~StreamScope() { castro_set_stream(saved); }
+};
+
+// A stage whose three directions are independent of one another: use(d) issues
+// direction d's launches on its own stream, between what is already on st and
+// what follows the stage there.  One direction's kernels fill the GPU only above
+// ~64^3 (256 blocks of 128 at 32^3, where a launch is all latency at a tenth of
+// the warps) and leave SMs idle in a last wave above.  The directions add into
+// arrays and scalars they share with atomics only.  Forward + backward on B200,
+// one stream -> three: 32^3 blast, 10 steps, 13.2 -> 9.5 ms; 64^3, 20 steps,
+// 78.4 -> 67.7 ms.
+struct Lanes {
+    castro_adj* a;
+    explicit Lanes(castro_adj* adj) : a(adj)
+    {
+        cudaEventRecord(a->ev_fork, a->st);
+        for (cudaStream_t l : a->lane) cudaStreamWaitEvent(l, a->ev_fork, 0);
+    }
+    cudaStream_t use(int d)
+    {
+        const cudaStream_t s = d == 0 ? a->st : a->lane[d - 1];
+        castro_set_stream(s);
+        g_part_lane = a->part[d];
+        return s;
+    }
+    ~Lanes()
+    {
+        for (int l = 0; l < 2; ++l) {
+            cudaEventRecord(a->ev_join[l], a->lane[l]);
+            cudaStreamWaitEvent(a->st, a->ev_join[l], 0);
+        }
+        castro_set_stream(a->st);
+        g_part_lane = nullptr;
+    }
+    Lanes(const Lanes&) = delete;
+    Lanes& operator=(const Lanes&) = delete;
 };
 
 // the working box and its grown boxes (Source/Castro_hydro.cpp:81-101)
@@ -1228,15 +1273,26 @@ void forward_step(castro_adj* a, double dt)
     divu(obx.lo, obx.hi, a->P->q.p, qbx.lo, qbx.hi, a->dx, a->P->div.p, obx.lo, obx.hi);
     double hdtdx[3], cdtdx[3];
     for (int d = 0; d < 3; ++d) { hdtdx[d] = 0.5 * dt / a->dx[d]; cdtdx[d] = dt / a->dx[d] / 3.0; }
-    for (int d = 0; d < 3; ++d)
+    // compute_flux's interface states, which nothing reads: one array per lane
+    // (the reverse arrays hold nothing yet)
+    double* const sink[3] = {a->P->qint.p, a->qlb[1].p, a->qlb[2].p};
+    {
+    Lanes lanes(a);
+    for (int d = 0; d < 3; ++d) {
+        lanes.use(d);
         trace_ppm(obx.lo, obx.hi, bx.lo, bx.hi, d + 1, a->P->q.p, qbx.lo, qbx.hi, a->P->qaux.p, qbx.lo, qbx.hi,
                   a->P->qm[d][d].p, a->P->qm[d][d].b.lo, a->P->qm[d][d].b.hi, a->P->qp[d][d].p, a->P->qp[d][d].b.lo,
                   a->P->qp[d][d].b.hi, bx.lo, bx.hi, a->dx, dt);
-    for (int d = 0; d < 3; ++d) {
         const IBx& b = a->tbx[d][d];
         compute_flux(b.lo, b.hi, a->P->qm[d][d].p, a->P->qm[d][d].b.lo, a->P->qm[d][d].b.hi, a->P->qp[d][d].p, a->P->qp[d][d].b.lo,
-                     a->P->qp[d][d].b.hi, a->P->F1[d].p, obx.lo, obx.hi, a->P->qint.p, obx.lo, obx.hi, a->P->G1[d].p, obx.lo,
+                     a->P->qp[d][d].b.hi, a->P->F1[d].p, obx.lo, obx.hi, sink[d], obx.lo, obx.hi, a->P->G1[d].p, obx.lo,
                      obx.hi, a->P->qaux.p, qbx.lo, qbx.hi, d + 1);
+    }
+    }
+    {
+    Lanes lanes(a);
+    for (int d = 0; d < 3; ++d) {
+        lanes.use(d);
         for (int tt = 0; tt < 2; ++tt) {
             int t = (tt == 0) ? (d == 0 ? 1 : 0) : (d == 2 ? 1 : 2);
             const IBx& tb = a->tbx[t][d];
@@ -1246,13 +1302,17 @@ void forward_step(castro_adj* a, double dt)
                    obx.hi, a->P->G1[d].p, obx.lo, obx.hi, cdtdx[d]);
         }
     }
+    }
+    {
+    Lanes lanes(a);
     for (int d = 0; d < 3; ++d) {
+        const cudaStream_t ls = lanes.use(d);
         int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
         for (int pp = 0; pp < 2; ++pp) {
             int x = pp == 0 ? t1 : t2, y = pp == 0 ? t2 : t1;
             const IBx& b = a->tbx[x][y];
             compute_flux(b.lo, b.hi, a->P->qm[x][y].p, a->P->qm[x][y].b.lo, a->P->qm[x][y].b.hi, a->P->qp[x][y].p,
-                         a->P->qp[x][y].b.lo, a->P->qp[x][y].b.hi, a->P->F2[x][y].p, obx.lo, obx.hi, a->P->qint.p, obx.lo, obx.hi,
+                         a->P->qp[x][y].b.lo, a->P->qp[x][y].b.hi, a->P->F2[x][y].p, obx.lo, obx.hi, sink[d], obx.lo, obx.hi,
                          a->P->G2[x][y].p, obx.lo, obx.hi, a->P->qaux.p, qbx.lo, qbx.hi, x + 1);
         }
         trans2(a->ebx[d].lo, a->ebx[d].hi, d + 1, t1 + 1, t2 + 1, a->P->qm[d][d].p, a->P->qm[d][d].b.lo, a->P->qm[d][d].b.hi,
@@ -1260,14 +1320,13 @@ void forward_step(castro_adj* a, double dt)
                obx.hi, a->P->qaux.p, qbx.lo, qbx.hi, a->P->F2[t1][t2].p, obx.lo, obx.hi, a->P->F2[t2][t1].p, obx.lo, obx.hi,
                a->P->G2[t1][t2].p, obx.lo, obx.hi, a->P->G2[t2][t1].p, obx.lo, obx.hi, hdtdx[d], hdtdx[t1], hdtdx[t2]);
         compute_flux(a->ebx[d].lo, a->ebx[d].hi, a->P->ql[d].p, obx.lo, obx.hi, a->P->qr[d].p, obx.lo, obx.hi,
-                     a->P->flux[d].p, a->gebx[d].lo, a->gebx[d].hi, a->P->qint.p, obx.lo, obx.hi, a->P->qe[d].p,
+                     a->P->flux[d].p, a->gebx[d].lo, a->gebx[d].hi, sink[d], obx.lo, obx.hi, a->P->qe[d].p,
                      a->gebx[d].lo, a->gebx[d].hi, a->P->qaux.p, qbx.lo, qbx.hi, d + 1);
-    }
-    for (int d = 0; d < 3; ++d) {
         apply_av(a->ebx[d].lo, a->ebx[d].hi, d + 1, a->dx, a->P->div.p, obx.lo, obx.hi, a->P->Sb.p, qbx.lo, qbx.hi,
                  a->P->flux[d].p, a->gebx[d].lo, a->gebx[d].hi);
-        copy(a->P->Fav[d], a->P->flux[d], st);
+        copy(a->P->Fav[d], a->P->flux[d], ls);
         normalize_species_fluxes(a->ebx[d].lo, a->ebx[d].hi, a->P->flux[d].p, a->gebx[d].lo, a->gebx[d].hi);
+    }
     }
     zero(a->P->src, st);                                          // hydro_source.setVal(0)
     fill_hydro_source(bx.lo, bx.hi, a->P->Sb.p, qbx.lo, qbx.hi, a->P->q.p, qbx.lo, qbx.hi, a->P->src.p, bx.lo, bx.hi,
@@ -1443,7 +1502,7 @@ void trans1_adj_zones(castro_adj* a, int d, int t, double cdtdx, double* cdtdxb)
         }
         st_rec<NS>(RF, i, j, k, frb);
         st_rec<NS>(LF, i, j, k, flb);
-        QAB(i, j, k, QGAMC) += gb;
+        aadd(&QAB(i, j, k, QGAMC), gb);
         return cb;
     }, cdtdxb);
 }
@@ -1499,7 +1558,7 @@ void trans2_adj_zones(castro_adj* a, int d, double c2, double c3, double* c2b, d
         st_rec<NS>(L2, i, j, k, f2lb);
         st_rec<NS>(R3, i, j, k, f3rb);
         st_rec<NS>(L3, i, j, k, f3lb);
-        QAB(i, j, k, QGAMC) += gb;
+        aadd(&QAB(i, j, k, QGAMC), gb);
         return make_double2(cb2, cb3);
     }, c2b, c3b);
 }
@@ -1605,18 +1664,18 @@ void reverse_step(castro_adj* a, double dt)
                                    a->dx[1], a->dx[2], a->fluxb[0].fab(), a->fluxb[1].fab(), a->fluxb[2].fab(),
                                    a->qeb[0].fab(), a->qeb[1].fab(), a->qeb[2].fab());
     adj_stage(a, "fill_hydro_source");
+    double hdtdx[3], cdtdx[3];
+    for (int d = 0; d < 3; ++d) { hdtdx[d] = 0.5 * dt / a->dx[d]; cdtdx[d] = dt / a->dx[d] / 3.0; }
+    {
+    Lanes lanes(a);
     for (int d = 0; d < 3; ++d) {
+        lanes.use(d);
         normalize_species_fluxes_adj_impl<NS>(a->ebx[d].lo, a->ebx[d].hi, a->P->Fav[d].fab(), a->fluxb[d].fab());
         apply_av_adj_impl<NS>(a->ebx[d].lo, a->ebx[d].hi, d, a->dx[d], a->P->div.fab(), a->P->Sb.fab(), a->fluxb[d].fab(),
                               a->divb.fab(), a->Sbb.fab());
         compute_flux_adj_impl<NS>(a->ebx[d].lo, a->ebx[d].hi, a->P->ql[d].fab(), a->P->qr[d].fab(), a->P->qaux.fab(),
                                   a->fluxb[d].fab(), a->qeb[d].fab(), a->qlb[d].fab(), a->qrb[d].fab(), a->qab.fab(), d,
                                   true);
-    }
-    adj_stage(a, "normalize/av/riemann3");
-    double hdtdx[3], cdtdx[3];
-    for (int d = 0; d < 3; ++d) { hdtdx[d] = 0.5 * dt / a->dx[d]; cdtdx[d] = dt / a->dx[d] / 3.0; }
-    for (int d = 0; d < 3; ++d) {
         int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
         trans2_adj_zones<NS>(a, d, hdtdx[t1], hdtdx[t2], sc + 6 + t1, sc + 6 + t2);
         IBx zb = a->ebx[d];
@@ -1625,37 +1684,47 @@ void reverse_step(castro_adj* a, double dt)
                            a->T2L[d][0].fab(), a->T2R[d][0].fab(), a->F2b[t1][t2].fab(), a->G2b[t1][t2].fab());
         gather_records<NS>(a->tbx[t2][t1], t2, zb, a->T2L[d][1].fab(), a->T2R[d][1].fab(), false, zb,
                            a->T2L[d][1].fab(), a->T2R[d][1].fab(), a->F2b[t2][t1].fab(), a->G2b[t2][t1].fab());
-    }
-    adj_stage(a, "trans2");
-    for (int x = 0; x < 3; ++x)
-        for (int y = 0; y < 3; ++y) {
-            if (x == y) continue;
+        for (int pp = 0; pp < 2; ++pp) {
+            const int x = pp == 0 ? t1 : t2, y = pp == 0 ? t2 : t1;
             compute_flux_adj_impl<NS>(a->tbx[x][y].lo, a->tbx[x][y].hi, a->P->qm[x][y].fab(), a->P->qp[x][y].fab(),
                                       a->P->qaux.fab(), a->F2b[x][y].fab(), a->G2b[x][y].fab(), a->qmb[x][y].fab(),
                                       a->qpb[x][y].fab(), a->qab.fab(), x, true);
         }
-    adj_stage(a, "riemann2");
+    }
+    }
+    adj_stage(a, "normalize/av/riemann3/trans2/riemann2");
+    {
+    // a lane per corrected direction t: its two launches add into the same face
+    // states, one after the other
+    Lanes lanes(a);
+    for (int t = 0; t < 3; ++t) {
+        lanes.use(t);
+        for (int d = 0; d < 3; ++d)
+            if (d != t) trans1_adj_zones<NS>(a, d, t, cdtdx[d], sc + 3 + d);
+    }
+    }
+    adj_stage(a, "trans1");
+    {
+    Lanes lanes(a);
     for (int d = 0; d < 3; ++d) {
+        lanes.use(d);
         const int ta = d == 0 ? 1 : 0, tb = d == 2 ? 1 : 2;
-        trans1_adj_zones<NS>(a, d, ta, cdtdx[d], sc + 3 + d);
-        trans1_adj_zones<NS>(a, d, tb, cdtdx[d], sc + 3 + d);
         IBx za = a->tbx[ta][d], zbb = a->tbx[tb][d];
         za.lo[ta] -= 1;
         zbb.lo[tb] -= 1;
         gather_records<NS>(a->tbx[d][d], d, za, a->T1L[d][ta].fab(), a->T1R[d][ta].fab(), true, zbb,
                            a->T1L[d][tb].fab(), a->T1R[d][tb].fab(), a->F1b[d].fab(), a->G1b[d].fab());
-    }
-    adj_stage(a, "trans1");
-    for (int d = 0; d < 3; ++d)
         compute_flux_adj_impl<NS>(a->tbx[d][d].lo, a->tbx[d][d].hi, a->P->qm[d][d].fab(), a->P->qp[d][d].fab(),
                                   a->P->qaux.fab(), a->F1b[d].fab(), a->G1b[d].fab(), a->qmb[d][d].fab(),
                                   a->qpb[d][d].fab(), a->qab.fab(), d);
-    adj_stage(a, "riemann1");
-    for (int d = 0; d < 3; ++d)
         trace_adj_impl<NS>(obx.lo, obx.hi, bx.lo, bx.hi, d, a->P->q.fab(), a->P->qaux.fab(), a->qmb[d][d].fab(),
-                           a->qpb[d][d].fab(), a->qb.fab(), a->qab.fab(), dt / a->dx[d], sc + d, a->flb.fab());
-    uflatten_adj_zones<NS>(obx.lo, obx.hi, a->P->q.fab(), a->P->qaux.fab(), a->qb.fab(), a->qab.fab(), a->flb.fab());
-    adj_stage(a, "trace");
+                           a->qpb[d][d].fab(), a->qb.fab(), a->qab.fab(), dt / a->dx[d], sc + d,
+                           d == 0 ? a->flb.fab() : a->qrb[d].fab());   // qrb is read no more
+    }
+    }
+    uflatten_adj_zones<NS>(obx.lo, obx.hi, a->P->q.fab(), a->P->qaux.fab(), a->qb.fab(), a->qab.fab(), a->flb.fab(),
+                           a->qrb[1].fab(), a->qrb[2].fab());
+    adj_stage(a, "riemann1/trace");
     divu_adj_impl<NS>(obx.lo, obx.hi, a->divb.fab(), a->qb.fab(), a->dx[0], a->dx[1], a->dx[2]);
     adj_stage(a, "divu");
     ctoprim_adj_impl<NS>(qbx.lo, qbx.hi, a->P->Sb.fab(), a->qb.fab(), a->qab.fab(), a->Sbb.fab());
@@ -2049,6 +2118,12 @@ castro_adj* castro_adj_create_window(const castro_instance_desc* desc, int nstep
     }
     a->P = &a->sets[0];
     ok = ok && cudaMalloc(&a->d_scal, 32 * sizeof(double)) == cudaSuccess;
+    // two doubles a block of the largest range a lane sums over (zones of the grown box)
+    const size_t part = 2 * ((size_t)nptsb(a->qbx) / 128 + 1);
+    for (double*& b : a->part) ok = ok && cudaMalloc(&b, part * sizeof(double)) == cudaSuccess;
+    for (cudaStream_t& l : a->lane) ok = ok && cudaStreamCreateWithFlags(&l, cudaStreamNonBlocking) == cudaSuccess;
+    ok = ok && cudaEventCreateWithFlags(&a->ev_fork, cudaEventDisableTiming) == cudaSuccess;
+    for (cudaEvent_t& e : a->ev_join) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaMalloc(&a->d_idx, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMalloc(&a->d_est, sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&a->d_chain, (nsteps + 2) * sizeof(double)) == cudaSuccess;
@@ -2101,6 +2176,13 @@ void castro_adj_destroy(castro_adj* a)
     if (a->d_idx) cudaFree(a->d_idx);
     if (a->d_est) cudaFree(a->d_est);
     if (a->d_chain) cudaFree(a->d_chain);
+    for (double* b : a->part)
+        if (b) cudaFree(b);
+    for (cudaStream_t l : a->lane)
+        if (l) cudaStreamDestroy(l);
+    if (a->ev_fork) cudaEventDestroy(a->ev_fork);
+    for (cudaEvent_t e : a->ev_join)
+        if (e) cudaEventDestroy(e);
     if (a->st) cudaStreamDestroy(a->st);
     delete a;
 }
