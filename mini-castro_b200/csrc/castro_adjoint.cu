@@ -977,8 +977,8 @@ struct StreamScope {
 // ~64^3 (256 blocks of 128 at 32^3, where a launch is all latency at a tenth of
 // the warps) and leave SMs idle in a last wave above.  The directions add into
 // arrays and scalars they share with atomics only.  Forward + backward on B200,
-// one stream -> three: 32^3 blast, 10 steps, 13.2 -> 9.5 ms; 64^3, 20 steps,
-// 78.4 -> 67.7 ms.
+// one stream -> three: 32^3 blast, 10 steps, 13.2 -> 9.1 ms; 64^3, 20 steps,
+// 78.4 -> 66.9 ms (the zeroing of the directions' arrays among it: 9.4, 67.6).
 struct Lanes {
     castro_adj* a;
     explicit Lanes(castro_adj* adj) : a(adj)
@@ -1620,16 +1620,20 @@ void reverse_step(castro_adj* a, double dt)
 {
     cudaStream_t st = a->st;
     const IBx &bx = a->bx, &obx = a->obx, &qbx = a->qbx;
+    {
+    Lanes lanes(a);
     for (Arr* r : {&a->Sbb, &a->qb, &a->qab, &a->divb, &a->srcb}) zero(*r, st);
     for (int d = 0; d < 3; ++d) {
+        const cudaStream_t ls = lanes.use(d);
         // F1b/G1b/F2b/G2b need no zeroing: the record gathers write every face
         // the Riemann adjoints read (the other components stay zero from creation)
         // qlb/qrb and the cross face states qmb/qpb[a][b] (a != b) are stored, not
         // accumulated, by their first writer (the riemann3 / riemann2 adjoints)
         // on exactly the faces their readers use
-        for (Arr* r : {&a->fluxb[d], &a->qeb[d]}) zero(*r, st);
-        zero(a->qmb[d][d], st);
-        zero(a->qpb[d][d], st);
+        for (Arr* r : {&a->fluxb[d], &a->qeb[d]}) zero(*r, ls);
+        zero(a->qmb[d][d], ls);
+        zero(a->qpb[d][d], ls);
+    }
     }
     double* sc = a->d_scal;
     adj_mark(a, "zero adjoint arrays");
