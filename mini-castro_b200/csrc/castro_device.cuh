@@ -114,8 +114,8 @@ CASTRO_HD double fminf_(double a, double b) { return (a < b) ? a : b; }
 // the truncated term of rcp is e^3, of root 5/16 e^3, beyond 2^-54; then the
 // rounding of the last step and, for root, half that of x * y).  128^3 step, 2
 // species, B200: 3368 -> 2992 us (trace 459 -> 332, riemann3 790 -> 685, front
-// 370 -> 310, update 440 -> 370); 64^3, 13 species: 1027 -> 885 us; error of a
-// step against 64-bit torch unchanged (profiles of the stages in castro_sim.cu).
+// 370 -> 310, update 440 -> 370); 64^3, 13 species: 1027 -> 885 us; a step
+// stays within 2e-15 (relative L2) of the same step in IEEE operations.
 // Arguments are normal numbers: the seeds flush subnormals, and a zero or an
 // infinity gives NaN where IEEE gives 0 or infinity.  Every denominator and
 // radicand here is bounded below by one of the floors above (root_floor takes
