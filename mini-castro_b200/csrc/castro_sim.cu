@@ -98,14 +98,16 @@ constexpr int TSEG = CASTRO_TRACE_SEG;   // zones of grow(bx,1) one trace thread
 #define CASTRO_R3_ROWS 1
 #endif
 // The 13-species instantiations carry larger records and take their own
-// register budgets (CASTRO_MINB13_*, 0 = the compiler's choice; measured on the
-// 13-species reference problem): the budgets tuned for 2 species make the
-// Riemann kernels spill.
+// register budgets (CASTRO_MINB13_*, 0 = the compiler's choice): the budgets
+// tuned for 2 species make the Riemann kernels spill.  64^3, 13 species, B200:
+// riemann2 at 3 / 4 / 5 blocks 205 / 193 / 283 us (168, 128, 96 registers; at 4 a
+// 16^3 box call is 93.3 us against 91.6, so it stays at 3), riemann3 with plain loads at the compiler's choice / 3 / 4 / 2 blocks 272 /
+// 184 / 234 / 197 us (180, 168, 128, 255 registers).
 #ifndef CASTRO_MINB13_EOS
 #define CASTRO_MINB13_EOS 4
 #endif
 #ifndef CASTRO_MINB13_R3
-#define CASTRO_MINB13_R3 0
+#define CASTRO_MINB13_R3 3
 #endif
 #ifndef CASTRO_MINB13_TRACE
 #define CASTRO_MINB13_TRACE 0
@@ -981,12 +983,11 @@ __global__ void LB_RIEMANN k_riemann2(SimDev S, const Work* wl)
 // Sborder values and the four divu nodes of apply_av) staged in shared memory
 // by cp.async; the cross-flux records stay plain loads served from L1
 // (measured on B200, 128^3, 2 species: 0 is faster, 637 against 657 us: the
-// 42 KB a block stages are taken from the L1 that serves the records).
+// 42 KB a block stages are taken from the L1 that serves the records).  13
+// species always load plainly: two blocks' slots fill the shared memory, and 64^3
+// took 219 us staged against 184 at three blocks.
 #ifndef CASTRO_R3_STAGE
 #define CASTRO_R3_STAGE 0
-#endif
-#ifndef CASTRO_R3_STAGE13
-#define CASTRO_R3_STAGE13 1
 #endif
 template <int NS>
 struct R3Slot {
@@ -997,10 +998,8 @@ struct R3Slot {
     static constexpr int DV = UB + 2 * NVAR;  // the four divu nodes of apply_av
     static constexpr int USED = DV + 4;
     static constexpr int STRIDE = USED | 1;   // odd: conflict-free 64-bit accesses
-    // 2 species: while four blocks fit; 13 species (255 registers, two blocks
-    // per SM either way): while two blocks fit
-    static constexpr int FIT = NS == 2 ? 4 : 2;
-    static constexpr bool ON = (NS == 2 ? CASTRO_R3_STAGE > 0 : CASTRO_R3_STAGE13 > 0) &&
+    static constexpr int FIT = 4;             // while four blocks fit
+    static constexpr bool ON = NS == 2 && CASTRO_R3_STAGE > 0 &&
                                STRIDE * BLOCK * 8 * FIT + FIT * 1024 <= 228 * 1024;
     static constexpr int BYTES = ON ? STRIDE * BLOCK * 8 : 0;
 };
