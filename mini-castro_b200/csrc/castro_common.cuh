@@ -33,13 +33,16 @@ struct NvtxRange {
 };
 
 // A FAB view in BL_FORT_FAB_ARG_3D form: Fortran order, component slowest.
-// The point within a component plane is numbered in 32 bits (a plane of 2^32
-// doubles would be 34 GB), the plane offset is 64-bit: a multiply-add per
-// component read, where 64-bit point arithmetic cost every access three wide
-// multiplications and the per-routine kernels and the adjoint's spent more
-// instructions on addresses than on FP64.  With range_point's 32-bit divisions
-// and clean_state in one launch, gradient of the 64^3, 20-step blast, B200:
-// 95.1 -> 85.7 ms; 32^3, 10 steps: 15.8 -> 14.6 ms.
+// The plane offset of a component is one multiply-add per read and the point
+// within the plane is shared by the components; numbered as one point of
+// nx ny nz ncomp every access cost three wide multiplications, and the
+// per-routine kernels and the adjoint's spent more instructions on addresses
+// than on FP64.  With range_point's 32-bit divisions and clean_state in one
+// launch, gradient of the 64^3, 20-step blast, B200: 95.1 -> 85.7 ms; 32^3, 10
+// steps: 15.8 -> 14.6 ms.  The point is a 64-bit number: a one-component array
+// of more than 2^32 points (34 GB) fits the GPU, and a 32-bit one would save no
+// more than 0.7% of that gradient (67.3 against 67.9 ms on three streams) and
+// nothing of a box call (88.9 against 89.3 us for 32^3).
 struct Fab {
     double* p;
     int lx, ly, lz;
@@ -47,7 +50,7 @@ struct Fab {
     size_t np;            // points of a component plane
     __host__ __device__ __forceinline__ double& operator()(int i, int j, int k, int n) const
     {
-        const unsigned t = (unsigned)(i - lx) + (unsigned)nx * ((unsigned)(j - ly) + (unsigned)ny * (unsigned)(k - lz));
+        const long long t = (i - lx) + (long long)nx * ((j - ly) + (long long)ny * (k - lz));
         return (p + t)[np * (unsigned)n];
     }
 };
