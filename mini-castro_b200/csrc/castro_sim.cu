@@ -161,7 +161,7 @@ struct Work {
 enum Region { R_VALID = 0, R_G1, R_G4, R_TBX, R_EBX, R_GHOST, R_SEG };
 
 // Points of a region are numbered in 32 bits (castro_sim_create rejects a
-// domain with a region of 2^31 points or more), components by 64-bit plane
+// region of 2^31 points or more that a sim's mode would number), components by 64-bit plane
 // offsets: one multiply-add per address, where 64-bit point numbers cost four
 // to six integer instructions for every double loaded or stored.
 struct Reg {
@@ -2661,6 +2661,7 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
     apply_table_l2_window(s->st);
     apply_table_l2_window(s->st2);
     const int NQS = 6 + ns, NTF = 7 + ns, NQF = 8 + ns, NV = 7 + ns;
+    const bool plain = mode == CASTRO_MODE_PLAIN || mode == CASTRO_MODE_PLAIN_BOX;
 
     long long oU = 0, oUb = 0, oQ = 0, oDiv = 0, oTr = 0, oF1 = 0, oF2 = 0, oFx = 0;
     std::vector<int> owner_all;
@@ -2706,7 +2707,12 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
         for (int a = 0; a < 3; ++a)
             for (int bb = 0; bb < 3; ++bb)
                 if (a != bb) { P.offF2[pair_index(a, bb)] = oF2; oF2 += npts_reg(P.lo, P.hi, R_TBX, 3 * a + bb) * NTF; }
-        if (npts_reg(P.lo, P.hi, R_G4, 0) > 2147483647LL - MAX_ITEM) {   // the largest region
+        // points are numbered in 32 bits: of the domain's regions in the modes that
+        // walk the domain (the grown one is the largest), of a box in the others
+        bool numbered = plain || npts_reg(P.lo, P.hi, R_G4, 0) <= 2147483647LL - MAX_ITEM;
+        for (int b = 0; plain && b < D.nbox; ++b)
+            numbered = numbered && npts_reg(D.box_lo + 3 * b, D.box_hi + 3 * b, R_VALID, 0) <= 2147483647LL - MAX_ITEM;
+        if (!numbered) {
             set_error(CASTRO_ERR_ARG, "castro_sim_create: a domain region exceeds 2^31 points");
             castro_sim_destroy(s);
             return nullptr;
@@ -2785,7 +2791,7 @@ castro_sim* castro_sim_create(int ninst, const castro_instance_desc* desc, int m
         if (ok && ns == 2 && column_tiles_on() && mode == CASTRO_MODE_BATCHED) ok = build_r23_work(s);
         if (ok && mode == CASTRO_MODE_PERSISTENT) ok = ns == 2 ? persistent_setup<2>(s) : persistent_setup<13>(s);
     }
-    if (ok && (mode == CASTRO_MODE_PLAIN || mode == CASTRO_MODE_PLAIN_BOX)) {
+    if (ok && plain) {
         long long nsb = 0, nsrc = 0, mx = 0;
         for (const BoxDev& B : s->hboxes) {
             s->offSb.push_back(nsb);
