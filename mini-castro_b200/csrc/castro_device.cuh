@@ -110,16 +110,25 @@ CASTRO_HD double fminf_(double a, double b) { return (a < b) ? a : b; }
 // that defines CASTRO_NR_ARITH (castro_sim.cu) takes these instead: the
 // hardware's ~20-bit seed refined by one third-order step of Newton's iteration
 // (Householder's family), straight-line, and one reciprocal for every division
-// by the same number.  Relative error at most 2^-52 (seed error below 2^-18:
-// the truncated term of rcp is e^3, of root 5/16 e^3, beyond 2^-54; then the
-// rounding of the last step and, for root, half that of x * y).  128^3 step, 2
-// species, B200: 3368 -> 2992 us (trace 459 -> 332, riemann3 790 -> 685, front
-// 370 -> 310, update 440 -> 370); 64^3, 13 species: 1027 -> 885 us; a step
-// stays within 2e-15 (relative L2) of the same step in IEEE operations.
+// by the same number.  With u = 2^-53 (an IEEE operation's error) and the seeds'
+// residual e below 2^-18 (of 1 - x y for rcp, of 1 - x y y for root): rcp is
+// within 1.5 u (the truncated e^3 below u / 2, the last rounding u), root
+// within 2 u (5/16 e^3 below u / 4, half the rounding of x y, the last
+// rounding), quot within 2.5 u (rcp and a product), root_floor within 2.5 u.
+// 128^3 step, 2 species, B200: 3368 -> 2992 us (trace 459 -> 332, riemann3
+// 790 -> 685, front 370 -> 310, update 440 -> 370); 64^3, 13 species: 1027 ->
+// 885 us; a step stays within 2e-15 (relative L2) of the same step in IEEE
+// operations.
 // Arguments are normal numbers: the seeds flush subnormals, and a zero or an
-// infinity gives NaN where IEEE gives 0 or infinity.  Every denominator and
-// radicand here is bounded below by one of the floors above (root_floor takes
-// the floor under the root) or is a state variable that is positive by then.
+// infinity gives NaN where IEEE gives 0 or infinity.  Most denominators and
+// radicands are bounded below by one of the floors above (root_floor takes the
+// floor under the root) or are positive for every state of the EOS table
+// (density, p, de/dT, gamma_1 p / rho, the sums over species).  Two are neither:
+// a transverse correction's density (trans1_state, trans2_state; tested for
+// being negative after its reciprocal is taken, which is then formed anew) --
+// exactly zero it leaves a face state without a velocity in either arithmetic,
+// infinite or NaN, and a NaN flux -- and the interface's rho e (riemann_cgf),
+// whose reciprocal feeds qgame alone, which no kernel of the step reads.
 // The exact build, the per-routine kernels and the adjoint keep IEEE / and sqrt.
 #if defined(CASTRO_NR_ARITH) && !defined(CASTRO_EXACT) && defined(__CUDA_ARCH__)
 #define CASTRO_NR 1
@@ -579,7 +588,11 @@ enum { EOS_RT = 1, EOS_RE = 2, EOS_RP = 3 };   // eos.F90:11-13
 // next solve starts converged instead of evaluating the EOS once more to find
 // a step of rounding size.  128^3 step, 2 species, B200: front 289 -> 222 us,
 // update 358 -> 291.  Where cleaning does change an argument (normalize_species clamps X at rho
-// below 1) the solve runs as always.  The exact build runs every solve.
+// below 1) the solve runs as always.  T is no further from the root than with
+// the extra evaluation, whose own rounding is larger than what the arguments
+// moved by: rms error of T over 50 (rho, T) cells on the Fermi-Dirac table 1e-16
+// .. 9.1e-13 (e / (T de/dT) = 0.2 .. 99) either way, the ratio of the two within
+// 0.5% in every cell.  The exact build runs every solve.
 struct EosKnown {
     double rho = 0.0, e = 0.0, abar = 0.0, zbar = 0.0;
     bool settled = false;
