@@ -33,6 +33,7 @@
 #include <sys/stat.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <numeric>
 #include <memory>
@@ -751,9 +752,8 @@ __global__ void LB_TRACE2 k_trace2(SimDev S, const Work* wl)
 }
 
 // Both passes in one launch, pass 2's items after pass 1's: the box entry
-// points' form while the two together are no more than one wave of pass 1's
-// blocks (three per SM), where a pass 2 launched behind pass 1 only adds its
-// latency
+// points' form while the two together are no more than one wave of its blocks
+// (trace_wave), where a pass 2 launched behind pass 1 only adds its latency
 template <int NS>
 __global__ void LB_TRACE k_trace_both(SimDev S, const Work* wl, int n)
 {
@@ -762,8 +762,33 @@ __global__ void LB_TRACE k_trace_both(SimDev S, const Work* wl, int n)
     else trace_item<NS, 2>(S, wl[blockIdx.x - n]);
 }
 
+// Blocks of k_trace_both that the current GPU holds at once (0 where that cannot
+// be had), looked up once per device.  B200: 444 for either species count, three
+// blocks of 128 threads (165 and 162 registers) on each of 148 SMs.
+template <int NS>
+int trace_wave()
+{
+    static std::atomic<int> wave[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int w = wave[dev].load(std::memory_order_relaxed);
+    if (w == 0) {
+        int sms = 0, per_sm = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_both<NS>, BLOCK, 0) != cudaSuccess)
+            return 0;
+        w = sms * per_sm;
+        wave[dev].store(w, std::memory_order_relaxed);
+    }
+    return w;
+}
+
 // whether the box entry points trace a box of n items a pass in one launch
-inline bool trace_in_one_launch(long long n) { return !CASTRO_TRACE_SPLIT || 2 * n <= 3 * 148; }
+template <int NS>
+bool trace_in_one_launch(long long n)
+{
+    return !CASTRO_TRACE_SPLIT || 2 * n <= trace_wave<NS>();
+}
 
 // compute_flux on the face (i,j,k) normal to D: left zone i-e_D, right zone i
 // returns (GDPRES, Godunov velocity normal to the face)
@@ -2563,7 +2588,7 @@ int step_impl(castro_sim* s)
         for (const BoxDev& B : s->hboxes) {
             long long nt = 0;
             for (int d = 0; d < 3; ++d) nt += (npts_reg(B.lo, B.hi, R_SEG, d) + BLOCK - 1) / BLOCK;
-            s->launches += 19 + (s->mode == CASTRO_MODE_PLAIN ? 36 : 6 + (trace_in_one_launch(nt) ? 1 : 2));
+            s->launches += 19 + (s->mode == CASTRO_MODE_PLAIN ? 36 : 6 + (trace_in_one_launch<NS>(nt) ? 1 : 2));
         }
         return castro_last_error();
     }
@@ -3457,7 +3482,7 @@ int box_hydro_launch(const BoxPlan& P, double* base, long long meta_doubles, con
     launch_behind(k_prep<NS>, nblocks[NL_G1], BLOCK, 0, cs, S, W + NLs.first[NL_G1]);
     if (!CASTRO_TRACE_SPLIT) {
         launch_behind(k_trace<NS>, nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE]);
-    } else if (trace_in_one_launch(nblocks[NL_TRACE])) {
+    } else if (trace_in_one_launch<NS>(nblocks[NL_TRACE])) {
         launch_behind(k_trace_both<NS>, 2 * nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE], nblocks[NL_TRACE]);
     } else {
         launch_behind(k_trace<NS>, nblocks[NL_TRACE], BLOCK, 0, cs, S, W + NLs.first[NL_TRACE]);
