@@ -221,6 +221,8 @@ __device__ __forceinline__ int ridx(const Reg& r, int i, int j, int k)
 // t / n for t < n + MAX_ITEM, m = div_mult(n): floor(2^32 / n) + 1 gives the
 // quotient exactly while t n < 2^32; beyond n = 2^15 the quotient is 0 or 1
 constexpr int MAX_ITEM = 1024;
+static_assert(BLOCK * CASTRO_R2_ROWS <= MAX_ITEM && BLOCK * CASTRO_R3_ROWS <= MAX_ITEM,
+              "an item's points past its first: what div_small's quotient is exact for");
 __host__ __device__ __forceinline__ unsigned div_mult(int n)
 {
     return (n == 1 || n > 32768) ? 0u : (unsigned)(4294967296ull / (unsigned)n) + 1u;
