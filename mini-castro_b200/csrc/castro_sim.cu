@@ -362,10 +362,11 @@ __device__ __forceinline__ double block_min(double m)
 // a stage's blocks may be placed on the SMs once every block of the stage
 // before has begun, so that the launch and the ramp of one stage lie under the
 // tail of the other; they touch nothing before that stage has completed
-// (griddepcontrol.wait waits for the whole grid and its writes).  A kernel
-// launched without the attribute runs straight through: the batched step keeps
-// its graph's ordinary edges, which measured faster there (16^3 66.7 us against
-// 70.2 with programmatic edges, 13 species 64^3 789 against 815, others equal).
+// (griddepcontrol.wait waits for the whole grid and its writes).  The kernels
+// that a box call and the batched step share run straight through when launched
+// without the attribute: the step keeps its graph's ordinary edges, which
+// measured faster there (16^3 66.7 us against 70.2 with programmatic edges, 13
+// species 64^3 789 against 815, others equal).
 __device__ __forceinline__ void stage_begin()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -418,7 +419,6 @@ __device__ __forceinline__ void front_body(const SimDev& S, const Work& w)
 template <int NS, bool COUL>
 __global__ void LB_EOS k_front(SimDev S, const Work* wl)
 {
-    stage_begin();
     front_body<NS, COUL>(S, wl[blockIdx.x]);
 }
 
@@ -481,7 +481,6 @@ __device__ __forceinline__ void ghost_body(const SimDev& S, const Work& w)
 template <int NS>
 __global__ void __launch_bounds__(BLOCK) k_ghost(SimDev S, const Work* wl)
 {
-    stage_begin();
     ghost_body<NS>(S, wl[blockIdx.x]);
 }
 
@@ -1492,7 +1491,6 @@ __device__ __forceinline__ void update_body(const SimDev& S, const Work& w)
 template <int NS, bool COUL>
 __global__ void LB_EOS k_update(SimDev S, const Work* wl)
 {
-    stage_begin();
     update_body<NS, COUL>(S, wl[blockIdx.x]);
 }
 
@@ -1555,7 +1553,6 @@ __device__ __forceinline__ void next_dt(InstState& st, int first)
 
 __global__ void k_dt(SimDev S, int ninst, int first)
 {
-    stage_begin();
     int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ninst) return;
     next_dt(S.st[n], first);
