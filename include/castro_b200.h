@@ -58,7 +58,8 @@ int         castro_last_error(void);          /* sticky: first error since castr
 void        castro_clear_error(void);
 const char* castro_error_string(void);
 int         castro_version(void);
-/* stream used by every launch (a cudaStream_t); default is the legacy stream 0 */
+/* stream used by every launch (a cudaStream_t); default is the legacy stream 0.
+ * It is the process's: host threads that use it share it */
 void        castro_set_stream(void* stream);
 void*       castro_get_stream(void);
 /* 1 when the library was built with CASTRO_EXACT (no FMA contraction, the
@@ -518,7 +519,10 @@ void fill_hydro_source_adj(const int* lo, const int* hi, const double* sourceb, 
  * The reverse sweep keeps a checkpoint every checkpoint_interval steps and
  * recomputes each segment; the time step's dependence on the state (CFL
  * reduction, 1.1x growth limit, stop-time clamp) is included.
- * desc->prob.pert (optional) must stay valid until the object is destroyed. */
+ * desc->prob.pert (optional) must stay valid until the object is destroyed.
+ * A call sets the process's library stream while it runs (and restores it), so
+ * the calls of two host threads, on one GPU or several, must not overlap with
+ * one another or with other calls on the library stream. */
 typedef struct castro_adj castro_adj;
 castro_adj* castro_adj_create(const castro_instance_desc* desc, int nsteps, int checkpoint_interval);
 /* The same with two more choices, for domains whose per-step arrays do not fit

@@ -158,8 +158,10 @@ __device__ __forceinline__ void aadd_tflux(const Fab& f, const Fab& qg, int i, i
 // their sum to the output scalar(s).
 constexpr int PART_MAX = 1 << 20;
 // PART_MAX x 2 doubles per device, allocated on first use on that device;
-// shared by every reduction of this library on the device, which are issued on
-// the library stream one after another
+// shared by the device's reductions that are issued on the library stream one
+// after another.  Those of a gradient's lanes run beside one another and have a
+// buffer per lane (castro_adj::part); the library stream and these pointers are
+// the process's, so the calls of two host threads must not overlap.
 constexpr int MAX_DEVICES = 64;
 double* g_part_dev[MAX_DEVICES] = {};
 double* g_part = nullptr;   // the current device's buffer (set by part_buffer)
@@ -407,9 +409,10 @@ void divu_adj_impl(const int* lo, const int* hi, Fab DIVB, Fab QB, double dx0, d
     });
 }
 
-// FLB: when given, the adjoint of the zone's flattening coefficient is left in
-// FLB (stored by direction 0, added by the others) for one uflatten reverse
-// after the three directions (uflatten_adj_zones); else it is reversed here
+// FLB: when given, this direction's adjoint of the zone's flattening coefficient
+// is stored there (each direction its own array, the directions run beside one
+// another) for one uflatten reverse of the three's sum (uflatten_adj_zones);
+// else it is reversed here
 template <int NS, int D>
 void trace_adj_dir(const int* lo, const int* hi, int vl, int vh, Fab Q, Fab QA, Fab QMB, Fab QPB, Fab QB, Fab QAB,
                    double dtdx, double* dtdxb, Fab FLB)

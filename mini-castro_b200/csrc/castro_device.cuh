@@ -1031,7 +1031,7 @@ CASTRO_HD void trace_project(const double I[3][4], double gam_g_ref, double un, 
                              double& un_o, double& rhoe_o, double& p_o);
 
 // One side's characteristic projection when it is not the usual case of
-// trace_states: trace_project with the integrals of the waves it reads
+// trace_segment: trace_project with the integrals of the waves it reads
 CASTRO_HD void trace_side(double rho_i, double un_i, double p_i, double re_i, double rho1, double p1, double re1, double uo,
                           double po, double gam, double un, double cc, bool plus, double& r, double& u, double& re, double& p)
 {

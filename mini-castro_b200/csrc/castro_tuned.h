@@ -5,7 +5,8 @@
 // per SM after the table: with 32-bit indices riemann1 / riemann2 fit seven
 // blocks (72 registers; 604 -> 566 us for riemann2 against five), and riemann3
 // without staging, one pass of faces per block and four blocks 637 us against
-// 657 staged with two passes.  Timing table of the autotuner (ms per step):
+// 657 staged with two passes.  Timing table of the autotuner (ms per step), made
+// with 64-bit indices and IEEE divisions: no row is the shape chosen below:
 //   block128_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    3.488
 //   block64_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    4.077
 //   block256_minbeos4_minbr30_minbriemann5_minbtrace3_minbtrace20_r2rows1_r2stage1_r3rows2_r3stage1_traceseg5_tracesplit1    4.852
