@@ -40,9 +40,9 @@ struct NvtxRange {
 // than on FP64.  With range_point's 32-bit divisions and clean_state in one
 // launch, gradient of the 64^3, 20-step blast, B200: 95.1 -> 85.7 ms; 32^3, 10
 // steps: 15.8 -> 14.6 ms.  The point is a 64-bit number: a one-component array
-// of more than 2^32 points (34 GB) fits the GPU, and a 32-bit one would save no
-// more than 0.7% of that gradient (67.3 against 67.9 ms on three streams) and
-// nothing of a box call (88.9 against 89.3 us for 32^3).
+// of more than 2^32 points (34 GB) fits the GPU, and a 32-bit one, which wraps
+// there, saves about 1% of that gradient (67.3 against 67.9-68.1 ms on three
+// streams) and nothing of a box call (88.9 against 89.3 us for 32^3).
 struct Fab {
     double* p;
     int lx, ly, lz;
